@@ -40,30 +40,20 @@
 
 namespace frep_math {
 
-FREP_HD double sin_poly(double r) {
-    /* r - r^3/3! + r^5/5! - ... - r^15/15!  (Horner in r^2) */
+/* The Taylor polynomials of sine and cosine, Horner in r^2:
+ *   r - r^3/3! + r^5/5! - ... - r^15/15!      (cosine: 1 - r^2/2! + ... + r^16/16!)
+ */
+FREP_HD double sincos_poly(double r, bool cosine) {
     const double r2 = r * r;
-    double p = -0x1.ae7f3e733b81fp-41;          /* -1/15! */
-    p = p * r2 + 0x1.6124613a86d09p-33;          /* +1/13! */
-    p = p * r2 - 0x1.ae64567f544e4p-26;          /* -1/11! */
-    p = p * r2 + 0x1.71de3a556c734p-19;          /* +1/9!  */
-    p = p * r2 - 0x1.a01a01a01a01ap-13;          /* -1/7!  */
-    p = p * r2 + 0x1.1111111111111p-7;           /* +1/5!  */
-    p = p * r2 - 0x1.5555555555555p-3;           /* -1/3!  */
-    return r + (r * r2) * p;
-}
-
-FREP_HD double cos_poly(double r) {
-    /* 1 - r^2/2! + r^4/4! - ... + r^16/16! */
-    const double r2 = r * r;
-    double p = 0x1.ae7f3e733b81fp-45;            /* +1/16! */
-    p = p * r2 - 0x1.93974a8c07c9dp-37;          /* -1/14! */
-    p = p * r2 + 0x1.1eed8eff8d898p-29;          /* +1/12! */
-    p = p * r2 - 0x1.27e4fb7789f5cp-22;          /* -1/10! */
-    p = p * r2 + 0x1.a01a01a01a01ap-16;          /* +1/8!  */
-    p = p * r2 - 0x1.6c16c16c16c17p-10;          /* -1/6!  */
-    p = p * r2 + 0x1.5555555555555p-5;           /* +1/4!  */
-    p = p * r2 - 0x1.0000000000000p-1;           /* -1/2!  */
+    double p = cosine ? 0x1.ae7f3e733b81fp-45 : -0x1.ae7f3e733b81fp-41;          /* +1/16! | -1/15! */
+    p = p * r2 + (cosine ? -0x1.93974a8c07c9dp-37 : 0x1.6124613a86d09p-33);      /* -1/14! | +1/13! */
+    p = p * r2 + (cosine ? 0x1.1eed8eff8d898p-29 : -0x1.ae64567f544e4p-26);      /* +1/12! | -1/11! */
+    p = p * r2 + (cosine ? -0x1.27e4fb7789f5cp-22 : 0x1.71de3a556c734p-19);      /* -1/10! | +1/9!  */
+    p = p * r2 + (cosine ? 0x1.a01a01a01a01ap-16 : -0x1.a01a01a01a01ap-13);      /* +1/8!  | -1/7!  */
+    p = p * r2 + (cosine ? -0x1.6c16c16c16c17p-10 : 0x1.1111111111111p-7);       /* -1/6!  | +1/5!  */
+    p = p * r2 + (cosine ? 0x1.5555555555555p-5 : -0x1.5555555555555p-3);        /* +1/4!  | -1/3!  */
+    if (!cosine) return r + (r * r2) * p;
+    p = p * r2 - 0x1.0000000000000p-1;                                           /* -1/2!  */
     return 1.0 + r2 * p;
 }
 
@@ -76,46 +66,43 @@ FREP_HD double reduce_pio2(double x, int* quadrant) {
     if (fabs(x) >= 1048576.0) {
         x = fmod(x, 0x1.921fb54442d18p+2); /* 2*pi rounded to double */
     }
-    const double k = floor(x * two_over_pi + 0.5);
+    const double t = x * two_over_pi + 0.5;
+#if defined(__CUDA_ARCH__)
+    /* floor(t) and its low bits for |t| < 2^51 without conversions: adding
+     * 1.5 * 2^52 rounds t to the nearest integer and leaves it in the low word */
+    const double m = t + 6755399441055744.0;
+    double k = m - 6755399441055744.0;
+    const bool above = k > t;
+    const int ki = __double2loint(m) - (above ? 1 : 0);
+    k = above ? k - 1.0 : k;
+#else
+    const double k = floor(t);
+    const int ki = (int)k;
+#endif
     double r = x - k * pio2_1;
     r = r - k * pio2_2;
     r = r - k * pio2_3;
-    const int ki = (int)k;
     *quadrant = ki & 3;
     return r;
 }
 
 }  // namespace frep_math
 
-FREP_HD float frep_sinf(float xf) {
+/* sin(x + quarter * pi/2): quarter 0 the sine, 1 the cosine. The quadrant picks
+ * the sine or the cosine polynomial's coefficients, not one of four branches:
+ * neighbouring lanes of a warp are often in different quadrants. */
+FREP_HD float frep_sin_quarter(float xf, int quarter) {
     const double x = (double)xf;
     if (!(fabs(x) < INFINITY)) return xf - xf; /* NaN for inf and NaN */
     int q;
     const double r = frep_math::reduce_pio2(x, &q);
-    double v;
-    switch (q) {
-        case 0: v = frep_math::sin_poly(r); break;
-        case 1: v = frep_math::cos_poly(r); break;
-        case 2: v = -frep_math::sin_poly(r); break;
-        default: v = -frep_math::cos_poly(r); break;
-    }
-    return (float)v;
+    q += quarter;
+    const double v = frep_math::sincos_poly(r, (q & 1) != 0);
+    return (float)((q & 2) ? -v : v);
 }
 
-FREP_HD float frep_cosf(float xf) {
-    const double x = (double)xf;
-    if (!(fabs(x) < INFINITY)) return xf - xf;
-    int q;
-    const double r = frep_math::reduce_pio2(x, &q);
-    double v;
-    switch (q) {
-        case 0: v = frep_math::cos_poly(r); break;
-        case 1: v = -frep_math::sin_poly(r); break;
-        case 2: v = -frep_math::cos_poly(r); break;
-        default: v = frep_math::sin_poly(r); break;
-    }
-    return (float)v;
-}
+FREP_HD float frep_sinf(float xf) { return frep_sin_quarter(xf, 0); }
+FREP_HD float frep_cosf(float xf) { return frep_sin_quarter(xf, 1); }
 
 FREP_HD float frep_expf(float xf) {
     const double x = (double)xf;
