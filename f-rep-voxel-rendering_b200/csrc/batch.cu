@@ -61,7 +61,7 @@ struct frep_batch {
     // plans: interval passes + point passes with 4 and 2 cells per lane
     frep::LevelPlan plan4{}, plan2{};
     uint32_t plan_slots = 0, plan_mm = 0;
-    bool plan_valid = false;
+    bool plan_valid = false, plan_exact = true;
     int interval_warps = 0, point_warps = 0;  // tuning hints (0 = automatic)
     // profiling (plain launches only): ev[0] before the root copy, ev[1] after
     // it, ev[2 + 3 l + kind] after level l's pass of that kind (0 interval,
@@ -204,7 +204,8 @@ frep_status ensure_keep(frep_batch* b, uint64_t words) {
 // What the level sequence needs to know about the batch's tapes.
 struct TapeStats {
     uint32_t slots = 4, mm = 1, longest = 1, max_levels = 0;
-    bool any_k4 = false, any_k2 = false;
+    uint64_t fine = 1;  // cells along an axis of the finest grid
+    bool any_k4 = false, any_k2 = false, pow2 = true;  // pow2: every last level's dim
 };
 
 frep_status check_tapes(const frep_batch* b, const frep_tape* const* tapes, TapeStats* st) {
@@ -220,22 +221,26 @@ frep_status check_tapes(const frep_batch* b, const frep_tape* const* tapes, Tape
         st->mm = std::max<uint32_t>(st->mm, t->ct.n_minmax);
         st->longest = std::max<uint32_t>(st->longest, (uint32_t)t->ct.instrs.size());
         st->max_levels = std::max<uint32_t>(st->max_levels, tr->grid.levels);
+        st->fine = std::max(st->fine, frep::fine_cells(tr->grid.dims, tr->grid.levels));
+        st->pow2 = st->pow2 && frep::pow2_dim(tr->grid.dims[tr->grid.levels - 1]);
         (tr->point_k == 4 ? st->any_k4 : st->any_k2) = true;
     }
     return FREP_OK;
 }
 
 frep_status ensure_plans(frep_batch* b, const TapeStats& st) {
-    if (b->plan_valid && b->plan_slots == st.slots && b->plan_mm == st.mm) return FREP_OK;
-    cudaError_t e = frep::plan_levels(st.slots, st.mm, 4, b->rounding, &b->plan4, b->interval_warps, b->point_warps);
+    const bool exact = st.fine <= 1ull << 24 && st.pow2;  // (what plan_levels asks of the grids)
+    if (b->plan_valid && b->plan_slots == st.slots && b->plan_mm == st.mm && b->plan_exact == exact) return FREP_OK;
+    cudaError_t e = frep::plan_levels(st.slots, st.mm, 4, b->rounding, &b->plan4, b->interval_warps, b->point_warps, 0, st.fine, st.pow2);
     if (e == cudaSuccess)
-        e = frep::plan_levels(st.slots, st.mm, 2, b->rounding, &b->plan2, b->interval_warps, b->point_warps);
+        e = frep::plan_levels(st.slots, st.mm, 2, b->rounding, &b->plan2, b->interval_warps, b->point_warps, 0, st.fine, st.pow2);
     if (e == cudaErrorInvalidValue)
         return fail(FREP_ERR_UNSUPPORTED, "frep_batch: %u slots / %u min-max ops exceed shared memory", st.slots, st.mm);
     if (e != cudaSuccess) return cuda_fail(e, "plan_levels");
     b->plan_valid = true;
     b->plan_slots = st.slots;
     b->plan_mm = st.mm;
+    b->plan_exact = exact;
     return FREP_OK;
 }
 
@@ -300,6 +305,8 @@ frep_status enqueue_voxelize(frep_batch* b, const uint8_t* d_area, const TapeSta
     a.n_trees = n;
     a.keep_scratch = b->keep;
     const frep::WarpScratch ws = batch_scratch(b, st);
+    a.longest = st.longest;
+    a.keep_words = (uint64_t)b->plan4.blocks * b->plan4.warps_per_block * ws.stride;
     a.keep_stride = ws.stride;
     a.mm_ofs = ws.mm_ofs;
     a.item_ofs = ws.item_ofs;
@@ -315,13 +322,13 @@ frep_status enqueue_voxelize(frep_batch* b, const uint8_t* d_area, const TapeSta
         if (e != cudaSuccess) return cuda_fail(e, "batched interval pass");
         if (prof) FREP_CUDA(cudaEventRecord(b->ev[2 + 3 * l], s));
         if (st.any_k4) {
-            e = frep::launch_level_scan(a, true, 4, s);
+            e = frep::launch_level_scan(a, true, frep::leaf_items(a, b->plan4), s);
             if (e == cudaSuccess) e = frep::launch_level(a, b->plan4, b->rounding, true, s);
             if (e != cudaSuccess) return cuda_fail(e, "batched point pass");
         }
         if (prof) FREP_CUDA(cudaEventRecord(b->ev[3 + 3 * l], s));
         if (st.any_k2) {
-            e = frep::launch_level_scan(a, true, 2, s);
+            e = frep::launch_level_scan(a, true, frep::leaf_items(a, b->plan2), s);
             if (e == cudaSuccess) e = frep::launch_level(a, b->plan2, b->rounding, true, s);
             if (e != cudaSuccess) return cuda_fail(e, "batched point pass");
         }
@@ -588,7 +595,8 @@ frep_status frep_batch_run(frep_batch* b, const frep_tape* const* tapes, const f
     std::vector<uint64_t> key = {L.total, n, st.slots, st.mm, st.longest, st.max_levels, st.any_k4, st.any_k2,
                                  fd.max_w, fd.max_h, fd.max_slots, (uint64_t)b->plan4.blocks,
                                  (uint64_t)b->plan4.warps_per_block, (uint64_t)b->plan4.point_warps_per_block,
-                                 (uint64_t)b->plan2.point_warps_per_block, (uint64_t)b->plan4.interval_ki,
+                                 (uint64_t)b->plan2.point_warps_per_block, (uint64_t)b->plan4.leaf_warps_per_block,
+                                 (uint64_t)b->plan4.leaf_blocks, (uint64_t)b->plan4.interval_ki,
                                  (uint64_t)level0_cells(b), (uint64_t)(uintptr_t)b->keep,
                                  (uint64_t)(uintptr_t)b->d_prefix, (uint64_t)(uintptr_t)A.d};
     for (uint32_t i = 0; i < n; i++) key.push_back(L.root_ofs[i]);
@@ -627,7 +635,10 @@ frep_status frep_batch_get_info(const frep_batch* b, frep_batch_info* info) {
     info->upload_bytes = b->last_upload;
     info->device_bytes = b->bytes;
     info->interval_warps_per_block = b->plan_valid ? (uint32_t)b->plan4.warps_per_block : 0;
-    info->point_warps_per_block = b->plan_valid ? (uint32_t)b->plan4.point_warps_per_block : 0;
+    info->point_warps_per_block =
+        !b->plan_valid ? 0
+                       : (uint32_t)(b->plan4.leaf_warps_per_block ? b->plan4.leaf_warps_per_block
+                                                                  : b->plan4.point_warps_per_block);
     info->root_cells_per_lane = b->plan_valid ? (uint32_t)level0_cells(b) : 0;
     return FREP_OK;
 }

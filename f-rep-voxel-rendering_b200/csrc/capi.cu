@@ -393,7 +393,9 @@ frep_status ensure_plan(frep_tree* tree, const frep_tape* tape, const char* who)
         tree->plan_round == tree->opts.rounding)
         return FREP_OK;
     const int k = tree->plain_k;
-    cudaError_t e = frep::plan_levels(n_slots, tape->ct.n_minmax, k, (int)tree->opts.rounding, &tree->plan);
+    cudaError_t e = frep::plan_levels(n_slots, tape->ct.n_minmax, k, (int)tree->opts.rounding, &tree->plan, 0, 0, 0,
+                                      frep::fine_cells(tree->grid.dims, tree->grid.levels),
+                                      frep::pow2_dim(tree->grid.dims[tree->grid.levels - 1]));
     if (e == cudaErrorInvalidValue)
         return fail(FREP_ERR_UNSUPPORTED, "%s: %u slots / %u min-max ops exceed shared memory", who, n_slots,
                     tape->ct.n_minmax);
@@ -427,6 +429,8 @@ frep_status enqueue_tree_levels(frep_tree* tree, const frep_tape* tape, float ta
     a.cursor = tree->d_cursor;
     a.n_trees = 1;
     a.keep_scratch = keep;
+    a.longest = (uint32_t)tape->ct.instrs.size();
+    a.keep_words = (uint64_t)plan.blocks * plan.warps_per_block * ws.stride;
     a.keep_stride = ws.stride;
     a.mm_ofs = ws.mm_ofs;
     a.item_ofs = ws.item_ofs;
@@ -441,7 +445,7 @@ frep_status enqueue_tree_levels(frep_tree* tree, const frep_tape* tape, float ta
         // Level 0 of one tree is one node: too few items to fill the GPU with
         // two cells per lane, so it keeps one (latency, not issue, bounds it).
         const int ki = l == 0 ? 1 : plan.interval_ki;
-        e = frep::launch_level_scan(a, point, point ? plan.point_k : ki, stream);
+        e = frep::launch_level_scan(a, point, point ? frep::leaf_items(a, plan) : ki, stream);
         if (e != cudaSuccess) return cuda_fail(e, "level_scan_kernel");
         e = frep::launch_level(a, plan, (int)tree->opts.rounding, point, stream, ki);
         if (e != cudaSuccess) return cuda_fail(e, "level kernel");
@@ -681,6 +685,7 @@ frep_status frep_tree_copy_tapes(frep_tree* tree, uint64_t* dst, uint64_t n_word
     if (n_words > tree->tape_cap) return fail(FREP_ERR_INVALID_ARG, "frep_tree_copy_tapes: beyond the pool");
     FREP_CUDA(cudaStreamSynchronize(tree->stream));
     FREP_CUDA(cudaMemcpy(dst, tree->tapes, n_words * 8, cudaMemcpyDeviceToHost));
+    frep::strip_marks(dst, n_words, frep::dev::TAPE_ALIGN_WORDS);  // the pools hold marked tapes
     return FREP_OK;
 }
 

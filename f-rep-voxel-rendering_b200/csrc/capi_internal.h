@@ -13,6 +13,7 @@
 #include "device_common.cuh"
 #include "frep.h"
 #include "kernels.h"
+#include "micro_ops.h"
 #include "tape_compiler.h"
 
 namespace frep {
@@ -58,11 +59,12 @@ void batch_host_ms(const frep_batch* b, double out[3]);
 
 struct frep_tape {
     frep::CompiledTape ct;
-    std::vector<uint64_t> record;  // [n_instr][instrs...] padded to 16 words
+    // [n_instr][instrs...] padded to 16 words, with the micro-op marks
+    std::vector<uint64_t> record;
     void build_record() {
         record.assign(frep::detail::align_up(1 + ct.instrs.size(), frep::dev::TAPE_ALIGN_WORDS), 0);
         record[0] = ct.instrs.size();
-        std::memcpy(&record[1], ct.instrs.data(), ct.instrs.size() * 8);
+        frep::mark_tape(ct.instrs.data(), (uint32_t)ct.instrs.size(), ct.n_slots, &record[1]);
     }
 };
 

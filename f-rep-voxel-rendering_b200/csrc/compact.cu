@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(256) tape_copy_kernel(const uint64_t* __restri
         if (!words) continue;
         const uint64_t* a = src + (size_t)s * TAPE_ALIGN_WORDS;
         uint64_t* b = dst + newofs[s];
-        for (uint32_t i = lane; i < words; i += 32) b[i] = a[i];
+        for (uint32_t i = lane; i < words; i += 32) b[i] = i ? a[i] & ~micro::MARKS : a[i];
     }
 }
 

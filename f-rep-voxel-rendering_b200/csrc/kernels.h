@@ -19,6 +19,9 @@ struct LevelLaunch {
     uint32_t n_trees;
     uint32_t level;
     uint32_t* keep_scratch;            // per-warp global scratch of the interval pass:
+    unsigned long long keep_words;     //   its size, u32 words (the last-level pass divides all of
+                                       //   it among its warps)
+    uint32_t longest;                  // instructions of the longest root tape
     uint32_t keep_stride;              //   u32 words per warp: keep masks [mm_ofs words,
     uint32_t mm_ofs;                   //   >= longest tape] then MIN/MAX choice masks
     uint32_t n_slots;                  // slot-file rows per lane (max over the batch)
@@ -30,6 +33,8 @@ struct LevelLaunch {
     uint32_t any_point_k;              // 1: a one-tree launch, whose last level runs with the
                                        //   launch's cells per lane whatever the tree's batch
                                        //   kind (TreeHeader::point_k); 0: only trees of that kind
+    uint32_t leaf_chunk;               // last-level pass: items per fetch at most, and a warp's share
+    uint32_t leaf_share;               //   of the scratch in 8-byte words (set by launch_level)
     uint32_t item_ofs;                 // per-warp scratch, u32 words: where the item tapes start
     uint32_t item_cap;                 //   and how many u64 words they may take (0 = no item
                                        //   pruning in the interval passes)
@@ -72,15 +77,51 @@ struct LevelPlan {
     int point_warps_per_block;
     int point_blocks;
     uint32_t point_smem_per_warp;
+    // last-level pass over micro-ops (tapes of at most 32 slots); 0 = the
+    // point pass above
+    int leaf_warps_per_block;
+    int leaf_blocks;
+    uint32_t leaf_smem_per_warp;
 };
+// How the last-level pass over micro-ops runs a launch. A warp's share of the
+// scratch holds the micro-ops of the longest tape (at most one per word); the
+// scratch of a few interval warps without item room holds fewer of those than
+// the pass has warps, and below half of them the point pass runs instead.
+struct LeafShape {
+    int blocks;      // 0: the point pass runs
+    uint32_t share;  // 8-byte words of scratch per warp
+};
+inline LeafShape leaf_shape(const LevelLaunch& a, const LevelPlan& p) {
+    if (!p.leaf_warps_per_block) return LeafShape{0, 0u};
+    const uint64_t longest = (a.longest + 2ull) & ~1ull, words8 = a.keep_words / 2, w = (uint64_t)p.leaf_warps_per_block;
+    uint64_t blocks = words8 / longest / w;
+    if (blocks > (uint64_t)p.leaf_blocks) blocks = (uint64_t)p.leaf_blocks;
+    if (2 * blocks < (uint64_t)p.leaf_blocks) return LeafShape{0, 0u};
+    const uint64_t share = words8 / (blocks * w) & ~1ull;
+    return LeafShape{(int)blocks, (uint32_t)(share < (1u << 24) ? share : 1u << 24)};
+}
+// `point_k` of launch_level_scan for a launch's last-level pass: its items.
+inline int leaf_items(const LevelLaunch& a, const LevelPlan& p) {
+    return leaf_shape(a, p).blocks ? -p.point_k : p.point_k;
+}
 
 // Cells per lane the point pass uses for a last level of this dim.
 int point_k_for(uint32_t dim);
 // interval_warps / point_warps: warps (tapes) per block, 0 = chosen from the
 // shared memory a warp needs, 1 or 4 = that many where shared memory allows.
 // interval_ki: cells per lane of the interval passes, 1 or 2 (0 = default).
+// fine_dim: the largest number of cells along an axis of a tree's finest grid;
+// pow2_leaves: every tree's last level has dim 4, 8, 16 or 32.
 cudaError_t plan_levels(uint32_t n_slots, uint32_t mm_cap, int point_k, int rounding, LevelPlan* plan,
-                        int interval_warps = 0, int point_warps = 0, int interval_ki = 0);
+                        int interval_warps = 0, int point_warps = 0, int interval_ki = 0, uint64_t fine_dim = 1,
+                        bool pow2_leaves = false);
+inline bool pow2_dim(uint32_t d) { return (d & (d - 1)) == 0; }
+// Cells along an axis of a grid's finest level (saturated at 2^40).
+inline uint64_t fine_cells(const uint32_t* dims, uint32_t levels) {
+    uint64_t f = 1;
+    for (uint32_t l = 0; l < levels; l++) f = f * dims[l] < (1ull << 40) ? f * dims[l] : 1ull << 40;
+    return f;
+}
 
 // Resets the headers of n trees (tape time from `tape_times`, or `tape_time`
 // when it is null) and writes their root nodes. Each tree's root tape must
@@ -94,7 +135,8 @@ cudaError_t launch_tree_init_staged(dev::TreeHeader* const* trees, uint32_t n, c
                                     const unsigned long long* offsets, const float* tape_times,
                                     cudaStream_t stream);
 // Work prefix of `level` over the batch, for interval (point = false) or
-// point passes with `point_k` cells per lane.
+// point passes with `point_k` cells per lane (leaf_items: negative for the
+// pass over micro-ops, of the trees of that batch kind).
 // out[3i..3i+2] = overflow flags, node words used, tape words used of tree i.
 cudaError_t launch_gather_usage(dev::TreeHeader* const* trees, uint32_t n, unsigned long long* out,
                                 cudaStream_t stream);

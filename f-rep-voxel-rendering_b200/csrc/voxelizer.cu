@@ -25,8 +25,12 @@
 // serves a whole batch of trees: a scan kernel lays the trees' items end to end
 // and a warp resolves each item to its tree (binary search, cached per warp),
 // so idle warps steal work from any scene of the batch.
+#include <algorithm>
+#include <type_traits>
+
 #include "device_common.cuh"
 #include "kernels.h"
+#include "micro_ops.h"
 
 namespace frep {
 namespace dev {
@@ -1527,11 +1531,13 @@ point_level_kernel(LevelLaunch p) {
     if (have_tree && lane == 0 && stat_work) atomicAdd(&T.H->cell_instr[L], stat_work);
 }
 
+#include "leaf_level.cuh"
+
 // Lays the batch's items for `level` end to end: prefix[i] = items of trees
 // before i that this launch serves (interval passes: trees for which `level`
 // is not the last; point passes: trees for which it is, with a last-level node
 // size that takes `k` cells per lane). An item is k mask words of a node (k
-// cells per lane). Interval passes also fix where each tree's next level
+// cells per lane), or for k < 0 one of the leaf pass (trees of batch kind -k). Interval passes also fix where each tree's next level
 // starts (node_ofs[level + 1]). One block.
 __device__ __forceinline__ unsigned long long level_items(TreeHeader* H, uint32_t L, int point, int k,
                                                           bool write_ofs, bool reuse, bool any_k) {
@@ -1540,12 +1546,13 @@ __device__ __forceinline__ unsigned long long level_items(TreeHeader* H, uint32_
     if ((point != 0) != last) return 0;
     const uint32_t dim = H->dims[L];
     const uint32_t words = dim * dim * dim / 32;
-    if (point && !any_k && H->point_k != (uint32_t)k) return 0;
+    const bool leaf = k < 0;
+    if (point && !any_k && H->point_k != (uint32_t)(leaf ? -k : k)) return 0;
     const uint32_t count = level_count(H, L, H->node_cap, H->node_size[L]);
     if (!point && write_ofs) H->node_ofs[L + 1] = H->node_ofs[L] + (unsigned long long)count * H->node_size[L];
     // with reuse, only the listed nodes are evaluated
     const uint32_t evaluated = reuse ? min(count, H->reuse_eval[L]) : count;
-    return (unsigned long long)evaluated * (words / (uint32_t)k);  // k: cells per lane of the pass
+    return (unsigned long long)evaluated * (leaf ? leaf_units(dim) : words / (uint32_t)k);
 }
 
 __global__ void __launch_bounds__(1024)
@@ -1724,6 +1731,8 @@ cudaError_t occupancy(Kern kernel, int threads, size_t smem, int* blocks) {
 // multiple of 8.
 int point_k_for(uint32_t dim) { return dev::point_k_of(dim); }
 
+constexpr uint32_t kLeafSlotBytes = 7168;  // slot rows per warp of the leaf pass
+
 template <int K>
 static cudaError_t plan_point(uint32_t n_slots, LevelPlan* plan, int warps_hint) {
     const uint32_t pt = (uint32_t)(n_slots * 32 * 4 * K + (dev::STAGE + 1) * 16 + 15) / 16 * 16;
@@ -1733,6 +1742,19 @@ static cudaError_t plan_point(uint32_t n_slots, LevelPlan* plan, int warps_hint)
     if (plan->point_warps_per_block == 4)
         return occupancy(dev::point_level_kernel<4, K>, 128, 4 * pt, &plan->point_blocks);
     return occupancy(dev::point_level_kernel<1, K>, 32, pt, &plan->point_blocks);
+}
+
+// The last-level pass over micro-ops takes every tape whose slots fit the row
+// mask, on grids whose last dims are powers of two and cell numbers exact floats. Rows for a warp: 20 warps to an SM (14 rows of 4 cells per lane, 28 of
+// 2), or what 2 cells per lane need for every slot of the batch.
+static cudaError_t plan_leaf(uint32_t n_slots, LevelPlan* plan, int warps_hint) {
+    static_assert(kLeafSlotBytes >= dev::LEAF_MIN_ROWS && kLeafSlotBytes % 16 == 0, "the decoder's constants fit");
+    const uint32_t rows = std::max<uint32_t>(kLeafSlotBytes, n_slots * 256);
+    const uint32_t smem = rows + dev::LEAF_FIXED_BYTES;
+    plan->leaf_smem_per_warp = smem;
+    plan->leaf_warps_per_block = warps_hint != 1 ? 4 : 1;
+    return plan->leaf_warps_per_block == 4 ? occupancy(dev::leaf_level_kernel<4>, 128, 4 * smem, &plan->leaf_blocks)
+                                           : occupancy(dev::leaf_level_kernel<1>, 32, smem, &plan->leaf_blocks);
 }
 
 template <int KI>
@@ -1748,7 +1770,7 @@ static cudaError_t plan_interval(bool four, int rounding, uint32_t iv, LevelPlan
 }
 
 cudaError_t plan_levels(uint32_t n_slots, uint32_t mm_cap, int point_k, int rounding, LevelPlan* plan,
-                        int interval_warps, int point_warps, int interval_ki) {
+                        int interval_warps, int point_warps, int interval_ki, uint64_t fine_dim, bool pow2_leaves) {
     (void)mm_cap;  // the choice masks live in global scratch
     // Two cells per lane halve the dispatch work per cell but double a warp's
     // slot rows: by default only while 16 warps still fit in an SM's shared
@@ -1779,6 +1801,11 @@ cudaError_t plan_levels(uint32_t n_slots, uint32_t mm_cap, int point_k, int roun
         e = ki == 2 ? plan_interval<2>(four, rounding, iv, plan) : plan_interval<1>(four, rounding, iv, plan);
     if (e != cudaSuccess) return e;
     plan->point_k = point_k;
+    plan->leaf_warps_per_block = 0;
+    if (n_slots <= dev::LEAF_MAX_SLOTS && fine_dim <= 1ull << 24 && pow2_leaves) {
+        e = plan_leaf(n_slots, plan, point_warps);
+        if (e != cudaSuccess) return e;
+    }
     if (point_k == 8) return plan_point<8>(n_slots, plan, point_warps);
     return point_k == 4 ? plan_point<4>(n_slots, plan, point_warps) : plan_point<2>(n_slots, plan, point_warps);
 }
@@ -1806,6 +1833,23 @@ cudaError_t launch_level_scan(const LevelLaunch& a, bool point, int point_k, cud
 
 cudaError_t launch_level(const LevelLaunch& a, const LevelPlan& plan, int rounding, bool point,
                          cudaStream_t stream, int interval_ki) {
+    const LeafShape leaf = point ? leaf_shape(a, plan) : LeafShape{0, 0u};
+    if (leaf.blocks) {
+        LevelLaunch b = a;
+        b.smem_per_warp = plan.leaf_smem_per_warp;
+        // Items per fetch at most: 128 dim-4 nodes, so that siblings that share a
+        // tape meet; of larger nodes, whose 256 cells per item share one already,
+        // 16, or 4 at level 1, where tapes have been shortened once and are long
+        // (128-scene batch: 14.1 ms with 32, 12.6 with 16, 9.0 with 8, 7.2 with 4;
+        // the 2048^3 scene's level 2: 2.04 ms with 32, 2.07 with 16, 2.27 with 4).
+        b.leaf_chunk = plan.point_k == 2 ? dev::LEAF_ITEMS : (a.level >= 2 ? 16u : 4u);
+        b.leaf_share = leaf.share;
+        const int w = plan.leaf_warps_per_block;
+        const size_t smem = (size_t)w * plan.leaf_smem_per_warp;
+        if (w == 4) dev::leaf_level_kernel<4><<<leaf.blocks, 128, smem, stream>>>(b);
+        else dev::leaf_level_kernel<1><<<leaf.blocks, 32, smem, stream>>>(b);
+        return cudaGetLastError();
+    }
     if (point) {
         LevelLaunch b = a;
         b.smem_per_warp = plan.point_smem_per_warp;
