@@ -280,7 +280,8 @@ int level0_cells(const frep_batch* b) {
 
 // The interval passes' per-warp scratch for the current set.
 frep::WarpScratch batch_scratch(const frep_batch* b, const TapeStats& st) {
-    return frep::warp_scratch(st.longest, st.mm, (uint32_t)b->plan4.interval_ki, b->rounding != 2);
+    return frep::warp_scratch(st.longest, st.mm, (uint32_t)b->plan4.interval_ki,
+                              b->rounding != 2 ? frep::kItemTapeWords : 0u);
 }
 
 // Enqueues the voxelization of every tree of the set: root copy + header

@@ -55,13 +55,16 @@ struct WarpScratch {
 // fit, the others run on the node's tape. (On the 128-scene batch, 1 MB per
 // warp executed exactly the same instructions.)
 constexpr uint32_t kItemTapeWords = 32768;
+// The least room that a single tree's passes prune items with (8 KB per warp).
+constexpr uint32_t kMinItemTapeWords = 1024;
 // ki: cells per lane of the interval pass (a keep mask and a choice-mask pair
-// per group of 32 cells). items: room for item tapes.
-inline WarpScratch warp_scratch(uint32_t longest, uint32_t mm_cap, uint32_t ki, bool items = false) {
+// per group of 32 cells). items: u64 words of room for item tapes at most (0:
+// no item pruning).
+inline WarpScratch warp_scratch(uint32_t longest, uint32_t mm_cap, uint32_t ki, uint32_t items = 0) {
     const uint32_t k = (ki * (longest ? longest : 1u) + 31u) / 32u * 32u;
     const uint32_t m = (2u * ki * (mm_cap ? mm_cap : 1u) + 31u) / 32u * 32u;
     const uint64_t want = 32ull * (longest ? longest : 1u);
-    const uint32_t ic = items ? (uint32_t)(want < kItemTapeWords ? (want + 15u) / 16u * 16u : kItemTapeWords) : 0u;
+    const uint32_t ic = (uint32_t)(want < items ? (want + 15u) / 16u * 16u : items);
     return WarpScratch{k + m + 2u * ic, k, k + m, ic};
 }
 

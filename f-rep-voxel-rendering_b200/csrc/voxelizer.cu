@@ -557,6 +557,14 @@ __device__ __noinline__ uint32_t prepare_items(const uint64_t* tape, uint32_t n,
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t dim = T.dim, ncx = T.ncx, ncy = T.ncy, ncz = T.ncz;
     const bool valid = lane < g;
+    // a tape with SIN / COS / EXP: the whole group runs the node's tape (found
+    // before anything is evaluated)
+    bool trans = false;
+    for (uint32_t i = lane; i < n; i += 32) {
+        const uint32_t op = w_op(__ldcg(&tape[i]));
+        trans |= op == OP_SIN || op == OP_COS || op == OP_EXP;
+    }
+    if (__any_sync(0xFFFFFFFFu, trans)) return 0u;
     // the item is a brick (brick_origin): its cells' bounding box
     uint32_t x0, y0, z0;
     brick_origin<KI>(grp + (valid ? lane : 0u), dim, T.dim_sh, &x0, &y0, &z0);
@@ -580,7 +588,7 @@ __device__ __noinline__ uint32_t prepare_items(const uint64_t* tape, uint32_t n,
         sts_iv<1>(lane_base + 3 * 32 * ROWB, b);
     }
     uint32_t mm = 0;
-    bool fin = true, trans = false;
+    bool fin = true;
     IVK<1> r;
     uint64_t pre[STAGE / 32];
     prefetch_chunk(pre, tape, 0, n, lane);
@@ -597,7 +605,6 @@ __device__ __noinline__ uint32_t prepare_items(const uint64_t* tape, uint32_t n,
                 const float c = __uint_as_float(d.y);
                 r.v[0] = make_float2(c, c);
             } else {
-                trans |= d.x == OP_SIN || d.x == OP_COS || d.x == OP_EXP;
                 r = iv_exec<ROUND, 1>(d, lane_base, lane, mmb, mm, mm_cap);
             }
             fin &= fabsf(r.v[0].x) <= 3.40282347e38f && fabsf(r.v[0].y) <= 3.40282347e38f;
@@ -605,7 +612,7 @@ __device__ __noinline__ uint32_t prepare_items(const uint64_t* tape, uint32_t n,
         }
     }
     __syncwarp();
-    if (trans || mm > mm_cap) return 0u;  // the whole group runs the node's tape
+    if (mm > mm_cap) return 0u;  // the whole group runs the node's tape
     const IVK<1> res = lds_iv<1>(lane_base);
     const bool empty = res.v[0].x > 0.0f, full = !empty && res.v[0].y < 0.0f;
     uint32_t plan = 0;
