@@ -408,6 +408,8 @@ frep_status frep_fit_pools(frep_ctx* ctx, const frep_tape* const* tapes, const f
                 o.tape_words = slot.second * 3 / 4 / 8;
                 st = frep_tree_create(ctx, &grids[i], &o, &slot.first);
                 if (st != FREP_OK) break;
+                // (one voxelization each: allocating the room would take longer)
+                slot.first->prune_items = false;
             }
             st = frep_voxelize(ctx, slot.first, tapes[i], tape_times ? tape_times[i] : 0.0f, nullptr);
             if (st != FREP_OK) break;

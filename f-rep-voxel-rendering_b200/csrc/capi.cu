@@ -509,19 +509,20 @@ frep_status voxelize_impl(frep_ctx* ctx, frep_tree* tree, const frep_tree* prev,
     // Per-warp scratch: a keep mask per instruction, a choice-mask pair per
     // MIN/MAX, and room for item tapes (item-level pruning): as much as is at
     // most a quarter of the tree's own pools and the context's budget holds,
-    // halving from the most down to 8 KB per warp (the items whose tapes do not
-    // fit run the node's tape); below that the passes run without item pruning
-    // (the same trees). Each tree keeps its scratch between voxelizations, so
-    // the bound keeps many small resident trees from each holding item room.
+    // from 32 down to 8 KB per warp (the items whose tapes do not fit run the
+    // node's tape); below that, and for tapes with transcendentals, which are
+    // not pruned, the passes run without item pruning (the same trees). Each
+    // tree keeps its scratch between voxelizations, so the bound keeps many
+    // small resident trees from each holding item room.
     // (The 2048^3 scene's fitted pools give 1,500 words per warp: its level-1
     // pass took 1.76 ms without item pruning, 1.27 with; a 75-primitive scene's
     // at 12 x 20 x 4 with 1,100 words 2.26 and 1.02 ms.)
     const uint64_t warps = (uint64_t)tree->plan.blocks * tree->plan.warps_per_block;
     const uint32_t ki = (uint32_t)tree->plan.interval_ki;
     frep::WarpScratch ws = frep::warp_scratch(n, tape->ct.n_minmax, ki);
-    if (tree->opts.rounding != FREP_ROUND_HYBRID) {
+    if (tree->opts.rounding != FREP_ROUND_HYBRID && !tape->transcendental && tree->prune_items) {
         const uint64_t room = (tree->node_cap * 4 + tree->tape_cap * 8) / 4 / 8 / warps;  // words per warp
-        uint32_t cap = (uint32_t)std::min<uint64_t>(room / 16 * 16, frep::kItemTapeWords);
+        uint32_t cap = (uint32_t)std::min<uint64_t>(room / 16 * 16, frep::kTreeItemTapeWords);
         for (; cap >= frep::kMinItemTapeWords; cap = cap / 2 / 16 * 16) {
             const frep::WarpScratch w = frep::warp_scratch(n, tape->ct.n_minmax, ki, cap);
             const bool fits = warps * w.stride <= tree->keep_words ||
@@ -532,8 +533,14 @@ frep_status voxelize_impl(frep_ctx* ctx, frep_tree* tree, const frep_tree* prev,
             break;
         }
     }
-    const uint64_t keep_words = warps * ws.stride;
+    uint64_t keep_words = warps * ws.stride;
     if (keep_words > tree->keep_words) {
+        // (a tree that sees ever longer tapes, as when pools are fitted, grows it
+        // by half at least, within the budget: each growth waits for the stream)
+        const uint64_t grown = tree->keep_words + tree->keep_words / 2;
+        if (grown > keep_words &&
+            ctx->used - std::min<uint64_t>(ctx->used, tree->keep_words * 4) + grown * 4 <= ctx->budget)
+            keep_words = grown;
         if (tree->keep) {
             cudaStreamSynchronize(tree->stream);
             cudaFree(tree->keep);

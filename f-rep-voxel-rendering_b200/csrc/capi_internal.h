@@ -61,7 +61,13 @@ struct frep_tape {
     frep::CompiledTape ct;
     // [n_instr][instrs...] padded to 16 words, with the micro-op marks
     std::vector<uint64_t> record;
+    bool transcendental = false;  // some instruction is SIN, COS or EXP
     void build_record() {
+        transcendental = false;
+        for (const uint64_t w : ct.instrs) {
+            const uint32_t op = frep::dev::w_op_host(w);
+            transcendental |= op == frep::dev::OP_SIN || op == frep::dev::OP_COS || op == frep::dev::OP_EXP;
+        }
         record.assign(frep::detail::align_up(1 + ct.instrs.size(), frep::dev::TAPE_ALIGN_WORDS), 0);
         record[0] = ct.instrs.size();
         frep::mark_tape(ct.instrs.data(), (uint32_t)ct.instrs.size(), ct.n_slots, &record[1]);
@@ -81,6 +87,7 @@ struct frep_tree {
     frep_voxelize_opts opts{};
     int point_k = 4;  // cells per lane of the last-level pass in batches (its batch kind, 4 or 2)
     int plain_k = 4;  // cells per lane of its own last-level passes (frep_voxelize and variants)
+    bool prune_items = true;  // its own passes may take room for item tapes
     bool external = false;  // header and pools live in caller-owned memory
     bool hdr_pending = false;              // external: header not yet written to the device
     frep::dev::TreeHeader pending_hdr{};   //   (write_tree_header)

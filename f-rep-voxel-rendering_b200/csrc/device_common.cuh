@@ -80,6 +80,7 @@ __host__ __device__ inline uint32_t node_words(uint32_t dim, bool last) {
 __device__ __constant__ const uint8_t kIntervalOps[16] = {0, 18, 18, 2, 2, 10, 16, 4, 4, 2, 0, 4, 0, 0, 0, 0};
 __device__ __constant__ const uint8_t kPointOps[16]    = {0, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 0, 0, 0, 0};
 
+inline uint32_t w_op_host(uint64_t w) { return (uint32_t)w & 0xFFu; }
 __device__ __forceinline__ uint32_t w_op(uint64_t w) { return (uint32_t)w & 0xFFu; }
 __device__ __forceinline__ uint32_t w_out(uint64_t w) { return ((uint32_t)w >> 16) & 0xFFFFu; }
 __device__ __forceinline__ uint32_t w_a(uint64_t w) { return (uint32_t)(w >> 32) & 0xFFFFu; }

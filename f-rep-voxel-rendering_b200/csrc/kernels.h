@@ -55,8 +55,9 @@ struct WarpScratch {
 // fit, the others run on the node's tape. (On the 128-scene batch, 1 MB per
 // warp executed exactly the same instructions.)
 constexpr uint32_t kItemTapeWords = 32768;
-// The least room that a single tree's passes prune items with (8 KB per warp).
-constexpr uint32_t kMinItemTapeWords = 1024;
+// The room that a single tree's passes prune items with: 8 to 32 KB per warp (a
+// new tree allocates it, 80 MB at most).
+constexpr uint32_t kMinItemTapeWords = 1024, kTreeItemTapeWords = 4096;
 // ki: cells per lane of the interval pass (a keep mask and a choice-mask pair
 // per group of 32 cells). items: u64 words of room for item tapes at most (0:
 // no item pruning).
@@ -76,6 +77,7 @@ struct LevelPlan {
     int blocks;                        // persistent grid
     uint32_t smem_per_warp;
     int interval_ki;                   // cells per lane in the interval passes (1 or 2)
+    bool micro;                        // the root level runs micro-ops (tapes of at most 32 slots)
     int point_k;                       // cells per lane in the point pass
     int point_warps_per_block;
     int point_blocks;

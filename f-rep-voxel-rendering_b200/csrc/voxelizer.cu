@@ -517,8 +517,298 @@ __device__ __forceinline__ void walk_lanes(const uint64_t* tape, uint32_t n, int
     }
 }
 
+// The same for a warp that has an SM (nearly) to itself, a single tree's root
+// level: the serial chain per instruction is one shuffle and the updates after
+// it, dead instructions go through it without a branch, and the next word is
+// fetched one instruction early (75 primitives: root level 0.69 -> 0.54 ms). Its
+// two loop bodies cost the levels below, with 16 warps per SM and more code
+// beside, more than they save (a batch's level 1 27.0 -> 29.1 ms).
+template <int KI, int S>
+__device__ __forceinline__ void walk_lanes_alone(const uint64_t* tape, uint32_t n, int mm, const uint2* mmb,
+                                           uint32_t* keep, const uint32_t (&ok_w)[KI], uint32_t lane,
+                                           uint32_t (&kept)[KI], uint32_t (&sig)[KI]) {
+    uint32_t lv[S][KI];
+#pragma unroll
+    for (int q = 0; q < S; q++)
+#pragma unroll
+        for (int h = 0; h < KI; h++) lv[q][h] = (q == 0 && lane == 0) ? ok_w[h] : 0u;  // slot 0: the result
+    bool plain = true;  // (the top chunk: mostly live)
+    int mm_top = mm;    // MIN/MAX instructions before the current chunk's end
+    for (int hi = (int)n; hi > 0; hi -= 32) {
+        const int lo = max(0, hi - 32);
+        const int m = hi - lo;
+        // lane j holds instruction lo + j (packed: out | a << 6 | b << 12 | reads
+        // a << 18 | reads b << 19 | MIN or MAX << 20) and, for a MIN/MAX, its choices
+        const uint64_t mine = (int)lane < m ? __ldcg(&tape[lo + lane]) : 0ull;
+        const uint32_t mop = w_op(mine);
+        const bool ism = (int)lane < m && is_mm(mop);
+        const uint32_t pk = (w_out(mine) & 63u) | (w_a(mine) & 63u) << 6 | (w_b(mine) & 63u) << 12 |
+                            (mop != OP_CONST ? 1u << 18 : 0u) | (is_binary(mop) ? 1u << 19 : 0u) | (ism ? 1u << 20 : 0u);
+        const uint32_t mball = __ballot_sync(0xFFFFFFFFu, ism);
+        const int mbase = mm_top - __popc(mball);
+        uint2 cb[KI];
+#pragma unroll
+        for (int h = 0; h < KI; h++)
+            cb[h] = ism ? mmb[(mbase + __popc(mball & lanemask_lt())) * KI + h] : make_uint2(0u, 0u);
+        uint32_t my_keep[KI], my_f[KI], my_s[KI];  // this lane's instruction: keep / chosen-input masks
+#pragma unroll
+        for (int h = 0; h < KI; h++) my_keep[h] = my_f[h] = my_s[h] = 0u;
+        int live = 0;  // instructions of this chunk live in some cell
+        int j = m - 1;
+        // instruction j (q: its packed word), live or not
+        auto step = [&](uint32_t q) {
+            const uint32_t o = q & 63u, a = (q >> 6) & 63u, b = (q >> 12) & 63u;
+            uint32_t k[KI], f[KI], sc[KI], anyk = 0;
+#pragma unroll
+            for (int h = 0; h < KI; h++) {
+                const uint32_t src = (S == 2 && o >= 32u) ? lv[S - 1][h] : lv[0][h];
+                k[h] = __shfl_sync(0xFFFFFFFFu, src, o & 31u);
+                anyk |= k[h];
+                f[h] = (q >> 18) & 1u ? k[h] : 0u;
+                sc[h] = (q >> 19) & 1u ? k[h] : 0u;
+            }
+            if ((q >> 20) & 1u) {
+#pragma unroll
+                for (int h = 0; h < KI; h++) {
+                    f[h] &= __shfl_sync(0xFFFFFFFFu, cb[h].x, j);
+                    sc[h] &= __shfl_sync(0xFFFFFFFFu, cb[h].y, j);
+                    if ((int)lane == j) {
+                        my_f[h] = f[h];
+                        my_s[h] = sc[h];
+                    }
+                }
+            }
+            live += anyk != 0u;
+            // clear the output slot, then set the inputs the choice uses
+            const bool at_o = lane == (o & 31u), at_a = lane == (a & 31u), at_b = lane == (b & 31u);
+#pragma unroll
+            for (int h = 0; h < KI; h++) {
+                if constexpr (S == 1) {
+                    lv[0][h] = (at_o ? 0u : lv[0][h]) | (at_a ? f[h] : 0u) | (at_b ? sc[h] : 0u);
+                } else {
+                    lv[0][h] = (at_o && o < 32u ? 0u : lv[0][h]) | (at_a && a < 32u ? f[h] : 0u) |
+                               (at_b && b < 32u ? sc[h] : 0u);
+                    lv[S - 1][h] = (at_o && o >= 32u ? 0u : lv[S - 1][h]) | (at_a && a >= 32u ? f[h] : 0u) |
+                                   (at_b && b >= 32u ? sc[h] : 0u);
+                }
+                if ((int)lane == j) my_keep[h] = k[h];
+            }
+        };
+        if (plain) {
+            uint32_t q = __shfl_sync(0xFFFFFFFFu, pk, j);
+            while (j >= 0) {
+                const uint32_t next = __shfl_sync(0xFFFFFFFFu, pk, (j - 1) & 31);  // (one instruction early)
+                step(q);
+                q = next;
+                j--;
+            }
+        } else {
+            while (j >= 0) {
+                uint32_t u0 = 0, u1 = 0;
+#pragma unroll
+                for (int h = 0; h < KI; h++) {
+                    u0 |= lv[0][h];
+                    if constexpr (S == 2) u1 |= lv[S - 1][h];
+                }
+                const uint64_t U = (uint64_t)__ballot_sync(0xFFFFFFFFu, u0 != 0u) |
+                                   (S == 2 ? (uint64_t)__ballot_sync(0xFFFFFFFFu, u1 != 0u) << 32 : 0ull);
+                const uint32_t cand = __ballot_sync(0xFFFFFFFFu, (int)lane <= j && ((U >> (pk & 63u)) & 1ull));
+                if (!cand) break;
+                j = 31 - __clz(cand);
+                step(__shfl_sync(0xFFFFFFFFu, pk, j));
+                j--;
+            }
+        }
+        plain = 2 * live >= m;  // the next chunk's mode, from this one's liveness
+        if ((int)lane < m) {
+            if constexpr (KI == 1) keep[lo + lane] = my_keep[0];
+            else reinterpret_cast<uint2*>(keep)[lo + lane] = make_uint2(my_keep[0], my_keep[1]);
+        }
+        // per cell: the chunk's kept instructions and MIN/MAX rewrites
+#pragma unroll
+        for (int h = 0; h < KI; h++) {
+            if (!__any_sync(0xFFFFFFFFu, my_keep[h] != 0u)) continue;
+            const uint32_t kc = transpose32(my_keep[h], lane);
+            kept[h] += __popc(kc);
+            uint32_t fc = 0, sc = 0;
+            if (__any_sync(0xFFFFFFFFu, (my_f[h] | my_s[h]) != 0u)) {
+                fc = transpose32(my_f[h], lane);
+                sc = transpose32(my_s[h], lane);
+            }
+            sig[h] = sig[h] * 0x9E3779B1u + (kc ^ (uint32_t)lo) * 0x85EBCA6Bu + fc * 0xC2B2AE35u + sc * 0x27D4EB2Fu;
+        }
+        mm_top = mbase;
+    }
+}
+
 // The forward loop's common opcodes as inline PTX with a jump table.
 #include "interval_dispatch.cuh"
+#include "interval_micro.cuh"
+
+// ---- forward pass over micro-ops ---------------------------------------------------
+//
+// The interval passes' forward evaluation as micro-ops (decode_single in
+// micro_ops.h: the next word's constant folded, results forwarded in registers,
+// renaming copies dropped; every MIN / MAX stays, in order, for its choices).
+// What bounds it is the interpreter: the loop over tape words loads both
+// operands of every word from shared memory, stores every result and spends 20
+// operations of two cells' MUL on glm's selects. Tapes of at most 32 slots.
+//
+// The root level runs them: long tapes, one after the other, nothing beside.
+// Per word of the 2048^3 scene's root tape (one cell per lane, a warp or two per
+// SM) 133 cycles instead of 307; two cells per lane in a batch of 128 (16 warps)
+// 201 instead of 262. Below the root, where a warp goes from one short tape to
+// the next through pruning, evaluation, the walk and the copies, the loop's 68
+// cases crowd the instruction cache: 521 cycles per word instead of 269, so those
+// levels keep the loop over words.
+
+// Decodes up to STAGE words from `from` on into stage[], slots replaced by row
+// offsets (rows of `stride` bytes), and the end mark. w: this lane's word of the
+// next 32 (loaded one block early); c: the two words before them. bad: some
+// constant is not finite.
+struct IvCarry {
+    uint32_t c1 = 0xFFFF0000u, c1_hi = 0u, c2 = 0xFFFF0000u;  // (before the tape: words that wrote no slot)
+};
+__device__ __forceinline__ void iv_micro_stage(const uint64_t* tape, uint32_t from, uint32_t n, uint4* stage,
+                                               uint32_t stride, uint32_t lane, uint64_t& w, IvCarry& c, bool& bad) {
+    uint32_t ops = 0;
+    const uint32_t end = min(n, from + STAGE);
+    __syncwarp();
+#pragma unroll 1
+    for (; from < end; from += 32) {
+        const uint64_t next = from + 32 + lane < n ? __ldcg(&tape[from + 32 + lane]) : 0ull;
+        const uint32_t lo = (uint32_t)w, hi = (uint32_t)(w >> 32);
+        uint32_t p1 = __shfl_up_sync(0xFFFFFFFFu, lo, 1), p1_hi = __shfl_up_sync(0xFFFFFFFFu, hi, 1);
+        uint32_t p2 = __shfl_up_sync(0xFFFFFFFFu, lo, 2);
+        if (lane == 0) {
+            p1 = c.c1;
+            p1_hi = c.c1_hi;
+            p2 = c.c2;
+        } else if (lane == 1) {
+            p2 = c.c1;
+        }
+        c.c1 = __shfl_sync(0xFFFFFFFFu, lo, 31);
+        c.c1_hi = __shfl_sync(0xFFFFFFFFu, hi, 31);
+        c.c2 = __shfl_sync(0xFFFFFFFFu, lo, 30);
+        const bool in = from + lane < n;
+        bad |= in && w_op(w) == OP_CONST && (hi & 0x7F800000u) == 0x7F800000u;
+        const bool there = in && !(lo & (uint32_t)micro::MARK_FOLD);
+        const bool gone = there && lane > 0 && micro::elided(w, p1);
+        const uint32_t kb = __ballot_sync(0xFFFFFFFFu, there && !gone), eb = __ballot_sync(0xFFFFFFFFu, gone);
+        const uint32_t renamed = __ffs(~(eb >> lane >> 1)) - 1u;  // elided words right after this one
+        const uint32_t dest = __shfl_sync(0xFFFFFFFFu, lo, (lane + renamed) & 31u);
+        if (there && !gone) {
+            uint32_t rows = 0;
+            const uint64_t u = micro::decode_single(
+                w, p1, p1_hi, ((p1 & (uint32_t)micro::MARK_FOLD) ? p2 : p1) >> 16, dest, &rows);
+            const uint32_t ul = (uint32_t)u, imm = (uint32_t)(u >> 32), x = ul & micro::MO_X;
+            const bool ia = micro::mo_kind_a(x) == micro::KIND_I || micro::mo_x_op(x) == micro::M_CONST;
+            stage[ops + __popc(kb & lanemask_lt())] =
+                make_uint4(ia ? imm : micro::mo_slot_a(ul) * stride,
+                           micro::mo_kind_b(x) == micro::KIND_I ? imm : micro::mo_slot_b(ul) * stride,
+                           micro::mo_slot_out(ul) * stride, x);
+        }
+        ops += __popc(kb);
+        w = next;
+    }
+    if (lane == 0) stage[ops] = make_uint4(0u, 0u, 0u, micro::M_END << 4);
+    __syncwarp();
+}
+
+// A slot row of the micro-op passes: lo0, lo1, hi0, hi1 (or lo, hi) per lane.
+template <int KI>
+__device__ __forceinline__ IVK<KI> lds_bounds(uint32_t a) {
+    IVK<KI> r;
+    if constexpr (KI == 1) {
+        r.v[0] = lds_f2(a);
+    } else {
+        const float4 t = lds_f4(a);
+        r.v[0] = make_float2(t.x, t.z);
+        r.v[1] = make_float2(t.y, t.w);
+    }
+    return r;
+}
+template <int KI>
+__device__ __forceinline__ void sts_bounds(uint32_t a, const IVK<KI>& r) {
+    if constexpr (KI == 1) sts_f2(a, r.v[0]);
+    else sts_f4(a, make_float4(r.v[0].x, r.v[1].x, r.v[0].y, r.v[1].y));
+}
+
+// One micro-op that the loop leaves to C++: any opcode and operand kinds.
+template <int ROUND, int KI>
+__device__ __noinline__ IvMicro<KI> iv_micro_rare(uint4 d, uint32_t lane_base, uint2* mmb, uint32_t mm_cap, IvMicro<KI> v) {
+    const uint32_t op = micro::mo_x_op(d.w), ka = micro::mo_kind_a(d.w), kb = micro::mo_kind_b(d.w);
+    IVK<KI> a, b;
+    if (ka == micro::KIND_S) a = lds_bounds<KI>(lane_base + d.x);
+    if (kb == micro::KIND_S) b = lds_bounds<KI>(lane_base + (micro::mo_binary(op) ? d.y : d.x));
+    const float ca = __uint_as_float(d.x), cb = __uint_as_float(d.y);
+    uint2 ch[KI];
+#pragma unroll
+    for (int h = 0; h < KI; h++) {
+        const float2 f = make_float2(v.lo[h], v.hi[h]);
+        const float2 x = ka == micro::KIND_S ? a.v[h] : (ka == micro::KIND_F ? f : make_float2(ca, ca));
+        const float2 y = kb == micro::KIND_S ? b.v[h] : (kb == micro::KIND_F ? f : make_float2(cb, cb));
+        const float2 r = iv_apply<ROUND>(op, 0ull, x, y);
+        if (is_mm(op)) {
+            const uint32_t c = mm_choice(op, x, y);
+            ch[h] = make_uint2(__ballot_sync(0xFFFFFFFFu, c & 1u), __ballot_sync(0xFFFFFFFFu, c & 2u));
+        }
+        v.lo[h] = r.x;
+        v.hi[h] = r.y;
+        v.s[h] = __fadd_rn(v.s[h], __fadd_rn(__fmul_rn(r.x, 0.0f), __fmul_rn(r.y, 0.0f)));
+    }
+    if (is_mm(op)) {
+        if ((threadIdx.x & 31) == 0 && v.mm < mm_cap) {
+#pragma unroll
+            for (int h = 0; h < KI; h++) mmb[v.mm * KI + h] = ch[h];
+        }
+        v.mm++;
+    }
+    if (!(d.w & micro::MO_NO_STORE)) {
+        IVK<KI> r;
+#pragma unroll
+        for (int h = 0; h < KI; h++) r.v[h] = make_float2(v.lo[h], v.hi[h]);
+        sts_bounds<KI>(lane_base + d.z, r);
+    }
+    return v;
+}
+
+// Evaluates a tape over this lane's boxes (in: X, Y, Z, T). v: the result's
+// bounds, the choices recorded, and per cell whether every bound was finite (s
+// = 0); the bounds and choices of a cell that had another are not the exact
+// path's. Returns false when some constant is not finite (nothing is evaluated).
+template <int ROUND, int KI>
+__device__ __forceinline__ bool iv_micro_forward(const uint64_t* tape, uint32_t n, const IVK<KI> (&in)[4], uint32_t lane,
+                                                 uint32_t lane_base, uint4* stage, uint32_t stride, uint2* mmb,
+                                                 uint32_t mm_cap, IvMicro<KI>& v) {
+    v.mm = 0;
+#pragma unroll
+    for (int h = 0; h < KI; h++) v.lo[h] = v.hi[h] = v.s[h] = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        sts_bounds<KI>(lane_base + k * stride, in[k]);
+#pragma unroll
+        for (int h = 0; h < KI; h++)
+            v.s[h] = __fadd_rn(v.s[h], __fadd_rn(__fmul_rn(in[k].v[h].x, 0.0f), __fmul_rn(in[k].v[h].y, 0.0f)));
+    }
+    IvCarry c;
+    bool bad = false;
+    uint64_t w = lane < n ? __ldcg(&tape[lane]) : 0ull;
+#pragma unroll 1
+    for (uint32_t from = 0; from < n; from += STAGE) {
+        iv_micro_stage(tape, from, n, stage, stride, lane, w, c, bad);
+        if (__any_sync(0xFFFFFFFFu, bad)) return false;
+        uint32_t at = smem_addr(stage);
+        while (true) {
+            at = iv_micro_run<ROUND, KI>(at, lane_base, mmb, mm_cap, v);
+            const uint4 d = lds_u4(at);
+            if (micro::mo_x_op(d.w) == micro::M_END) break;
+            v = iv_micro_rare<ROUND, KI>(d, lane_base, mmb, mm_cap, v);
+            at += 16;
+        }
+    }
+    return true;
+}
 
 // ---- item-level pruning (this library's addition) ----------------------------------
 //
@@ -575,18 +865,14 @@ __device__ __noinline__ uint32_t prepare_items(const uint64_t* tape, uint32_t n,
     const uint32_t glo[3] = {ncx * dim + x0, ncy * dim + y0, ncz * dim + z0};
     const uint32_t ghi[3] = {ncx * dim + x1, ncy * dim + y1, ncz * dim + z1};
     const float low[3] = {T.lx, T.ly, T.lz};
+    IVK<1> in[4];
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-        IVK<1> b;
-        b.v[0] = make_float2(__fadd_rn(low[k], __fmul_rn((float)glo[k], cs)),
-                             __fadd_rn(__fadd_rn(low[k], __fmul_rn((float)ghi[k], cs)), cs));
-        sts_iv<1>(lane_base + k * 32 * ROWB, b);
-    }
-    {
-        IVK<1> b;
-        b.v[0] = make_float2(T.tt, T.tt);
-        sts_iv<1>(lane_base + 3 * 32 * ROWB, b);
-    }
+    for (int k = 0; k < 3; k++)
+        in[k].v[0] = make_float2(__fadd_rn(low[k], __fmul_rn((float)glo[k], cs)),
+                                 __fadd_rn(__fadd_rn(low[k], __fmul_rn((float)ghi[k], cs)), cs));
+    in[3].v[0] = make_float2(T.tt, T.tt);
+#pragma unroll
+    for (int k = 0; k < 4; k++) sts_iv<1>(lane_base + k * 32 * ROWB, in[k]);
     uint32_t mm = 0;
     bool fin = true;
     IVK<1> r;
@@ -611,9 +897,9 @@ __device__ __noinline__ uint32_t prepare_items(const uint64_t* tape, uint32_t n,
             sts_iv<1>(lane_base + d.w, r);
         }
     }
+    const IVK<1> res = lds_iv<1>(lane_base);
     __syncwarp();
     if (mm > mm_cap) return 0u;  // the whole group runs the node's tape
-    const IVK<1> res = lds_iv<1>(lane_base);
     const bool empty = res.v[0].x > 0.0f, full = !empty && res.v[0].y < 0.0f;
     uint32_t plan = 0;
     if (valid && fin && empty) plan = 2;
@@ -684,7 +970,7 @@ __device__ __noinline__ uint32_t prepare_items(const uint64_t* tape, uint32_t n,
 // (KI words per instruction) | choice masks (KI uint2 per MIN/MAX): they grow
 // with the tape, and in shared memory they would cap the resident warps for
 // every tree of a batch at what its longest tape allows.
-template <int ROUND, int WARPS, int KI>
+template <int ROUND, int WARPS, int KI, bool MO>
 // At least 16 warps per SM (4 blocks of 4 or 16 of 1): up to 128 registers.
 // Shared memory already limits a batch's plan to about 16 resident warps, and
 // a cap of 96 registers spills inside the forward pass: on a 128-scene batch
@@ -692,7 +978,7 @@ template <int ROUND, int WARPS, int KI>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 4 : 16)
 interval_level_kernel(LevelLaunch p) {
     extern __shared__ __align__(16) unsigned char smem[];
-    static_assert(ROUND != 2 || KI == 1, "the hybrid affine mode runs one cell per lane");
+    static_assert(ROUND != 2 || (KI == 1 && !MO), "the hybrid affine mode runs one cell per lane, word by word");
     // bytes per lane per slot: KI intervals; the hybrid mode's 8 floats (lo, hi,
     // c, x | y, z, e, 0) as two conflict-free half rows of 16 bytes per lane
     constexpr uint32_t ROWB = ROUND == 2 ? 32 : 8 * KI;
@@ -737,8 +1023,9 @@ interval_level_kernel(LevelLaunch p) {
     // (not at level 0: with bricks, a batch's root level pruned per brick, a
     // dozen bricks per fetch, took 74.7 ms against 43.0 ms without)
     uint64_t* items = nullptr;
-    if constexpr (ROUND < 2)
+    if constexpr (ROUND < 2 && !MO)
         if (p.item_cap && L > 0) items = reinterpret_cast<uint64_t*>(keep + p.item_ofs);
+    const uint64_t* exact_tape = nullptr;  // a tape whose bounds were not all finite
     // (the items pg_first .. pg_first + pg_g - 1, consecutive in this warp's
     // fetches; this lane's plan is item pg_first + lane's)
     unsigned long long pg_first = 0;
@@ -786,7 +1073,7 @@ interval_level_kernel(LevelLaunch p) {
                 }
             }
 
-            if constexpr (ROUND < 2) {
+            if constexpr (ROUND < 2 && !MO) {
                 if (items && 32u * KI < dim * dim * dim) {
                     if (item - pg_first >= pg_g) {
                         // the rest of this node's items in the fetched chunk, up to 32
@@ -828,7 +1115,25 @@ interval_level_kernel(LevelLaunch p) {
                 bt.v[h] = make_float2(T.tt, T.tt);
             }
             uint32_t mm = 0;
-            IVK<KI> r;
+            IVK<KI> r, res;
+            bool exact = true;  // the exact path runs
+            if constexpr (MO) {
+                if (tape != exact_tape) {
+                    IvMicro<KI> v;
+                    const IVK<KI> in[4] = {bx, by, bz, bt};
+                    bool ok = iv_micro_forward<ROUND, KI>(tape, n, in, lane, lane_base, stage, 32 * ROWB, mmb, p.mm_cap, v);
+#pragma unroll
+                    for (int h = 0; h < KI; h++) {
+                        ok = ok && v.s[h] == 0.0f;
+                        res.v[h] = make_float2(v.lo[h], v.hi[h]);
+                    }
+                    mm = v.mm;
+                    exact = !__all_sync(0xFFFFFFFFu, ok);
+                    if (exact) exact_tape = tape;  // (its next items take the exact path at once)
+                }
+            }
+            if (exact) {
+            mm = 0;
             uint64_t pre[STAGE / 32];
             prefetch_chunk(pre, tape, 0, n, lane);
             if constexpr (ROUND == 2) {
@@ -893,7 +1198,7 @@ interval_level_kernel(LevelLaunch p) {
                 prefetch_chunk(pre, tape, base + STAGE, n, lane);
                 __syncwarp();
                 const uint32_t sbase = smem_addr(stage);
-                if constexpr (KI == 2) {
+                if constexpr (KI == 2 && !MO) {
                     uint32_t j = 0;
                     while (true) {
                         IvRun run;
@@ -925,12 +1230,13 @@ interval_level_kernel(LevelLaunch p) {
                 }
             }
             }
+            res = lds_iv<KI>(lane_base);
+            }
             __syncwarp();
             // the reference's work: every cell evaluates its node's tape
             stat_work += 32ull * KI * n_node;
 
             // ---- classification (voxelizer/main.comp:88-108) ----
-            const IVK<KI> res = lds_iv<KI>(lane_base);
             uint32_t leaf_w[KI], amb_w[KI], ok_w[KI];
             bool ok[KI];
             unsigned long long my_child[KI];
@@ -997,7 +1303,8 @@ interval_level_kernel(LevelLaunch p) {
                 if (p.n_slots <= 32) {
                     // live sets spread over the lanes' registers: no shared
                     // memory on the walk's path
-                    walk_lanes<KI, 1>(tape, n, (int)mm, mmb, keep, ok_w, lane, kept, sig);
+                    if constexpr (MO && KI == 1) walk_lanes_alone<1, 1>(tape, n, (int)mm, mmb, keep, ok_w, lane, kept, sig);
+                    else walk_lanes<KI, 1>(tape, n, (int)mm, mmb, keep, ok_w, lane, kept, sig);
                 } else if (p.n_slots <= 64) {
                     walk_lanes<KI, 2>(tape, n, (int)mm, mmb, keep, ok_w, lane, kept, sig);
                 } else {
@@ -1764,16 +2071,29 @@ static cudaError_t plan_leaf(uint32_t n_slots, LevelPlan* plan, int warps_hint) 
                                            : occupancy(dev::leaf_level_kernel<1>, 32, smem, &plan->leaf_blocks);
 }
 
-template <int KI>
+template <int KI, bool MO>
 static cudaError_t plan_interval(bool four, int rounding, uint32_t iv, LevelPlan* plan) {
-    if (rounding == 2)
-        return four ? occupancy(dev::interval_level_kernel<2, 4, 1>, 128, 4 * iv, &plan->blocks)
-                    : occupancy(dev::interval_level_kernel<2, 1, 1>, 32, iv, &plan->blocks);
     if (four)
-        return rounding ? occupancy(dev::interval_level_kernel<1, 4, KI>, 128, 4 * iv, &plan->blocks)
-                        : occupancy(dev::interval_level_kernel<0, 4, KI>, 128, 4 * iv, &plan->blocks);
-    return rounding ? occupancy(dev::interval_level_kernel<1, 1, KI>, 32, iv, &plan->blocks)
-                    : occupancy(dev::interval_level_kernel<0, 1, KI>, 32, iv, &plan->blocks);
+        return rounding ? occupancy(dev::interval_level_kernel<1, 4, KI, MO>, 128, 4 * iv, &plan->blocks)
+                        : occupancy(dev::interval_level_kernel<0, 4, KI, MO>, 128, 4 * iv, &plan->blocks);
+    return rounding ? occupancy(dev::interval_level_kernel<1, 1, KI, MO>, 32, iv, &plan->blocks)
+                    : occupancy(dev::interval_level_kernel<0, 1, KI, MO>, 32, iv, &plan->blocks);
+}
+static cudaError_t plan_interval(int ki, bool four, int rounding, uint32_t iv, LevelPlan* plan) {
+    if (rounding == 2)
+        return four ? occupancy(dev::interval_level_kernel<2, 4, 1, false>, 128, 4 * iv, &plan->blocks)
+                    : occupancy(dev::interval_level_kernel<2, 1, 1, false>, 32, iv, &plan->blocks);
+    if (plan->micro) {  // (the root level's kernel; its grid is that of the others)
+        const cudaError_t e = ki == 2 ? plan_interval<2, true>(four, rounding, iv, plan)
+                                      : plan_interval<1, true>(four, rounding, iv, plan);
+        if (e != cudaSuccess) return e;
+        const int blocks = plan->blocks;
+        const cudaError_t e2 = ki == 2 ? plan_interval<2, false>(four, rounding, iv, plan)
+                                       : plan_interval<1, false>(four, rounding, iv, plan);
+        plan->blocks = std::min(plan->blocks, blocks);
+        return e2;
+    }
+    return ki == 2 ? plan_interval<2, false>(four, rounding, iv, plan) : plan_interval<1, false>(four, rounding, iv, plan);
 }
 
 cudaError_t plan_levels(uint32_t n_slots, uint32_t mm_cap, int point_k, int rounding, LevelPlan* plan,
@@ -1803,9 +2123,9 @@ cudaError_t plan_levels(uint32_t n_slots, uint32_t mm_cap, int point_k, int roun
     // Both cell widths may run with this plan's shared memory (a level-0 pass
     // takes one cell per lane): raise both kernels' limits, then size the grid
     // for the planned width.
-    cudaError_t e = ki == 2 ? plan_interval<1>(four, rounding, iv, plan) : plan_interval<2>(four, rounding, iv, plan);
-    if (e == cudaSuccess)
-        e = ki == 2 ? plan_interval<2>(four, rounding, iv, plan) : plan_interval<1>(four, rounding, iv, plan);
+    plan->micro = n_slots <= micro::MO_SLOTS && rounding != 2;
+    cudaError_t e = plan_interval(3 - ki, four, rounding, iv, plan);
+    if (e == cudaSuccess) e = plan_interval(ki, four, rounding, iv, plan);
     if (e != cudaSuccess) return e;
     plan->point_k = point_k;
     plan->leaf_warps_per_block = 0;
@@ -1879,27 +2199,32 @@ cudaError_t launch_level(const LevelLaunch& a, const LevelPlan& plan, int roundi
     const int w = plan.warps_per_block;
     const size_t smem = (size_t)w * plan.smem_per_warp;
     const int tpb = 32 * w;
-#define FREP_IV_LAUNCH(R, W, KI) dev::interval_level_kernel<R, W, KI><<<plan.blocks, tpb, smem, stream>>>(b)
-    if (rounding == 2) {
-        if (w == 4) FREP_IV_LAUNCH(2, 4, 1);
-        else FREP_IV_LAUNCH(2, 1, 1);
-    } else if ((interval_ki ? interval_ki : plan.interval_ki) == 2) {
-        if (w == 4) {
-            if (rounding) FREP_IV_LAUNCH(1, 4, 2);
-            else FREP_IV_LAUNCH(0, 4, 2);
-        } else {
-            if (rounding) FREP_IV_LAUNCH(1, 1, 2);
-            else FREP_IV_LAUNCH(0, 1, 2);
-        }
-    } else {
-        if (w == 4) {
-            if (rounding) FREP_IV_LAUNCH(1, 4, 1);
-            else FREP_IV_LAUNCH(0, 4, 1);
-        } else {
-            if (rounding) FREP_IV_LAUNCH(1, 1, 1);
-            else FREP_IV_LAUNCH(0, 1, 1);
-        }
+#define FREP_IV_LAUNCH(R, W, KI, MO) dev::interval_level_kernel<R, W, KI, MO><<<plan.blocks, tpb, smem, stream>>>(b)
+#define FREP_IV_ROUND(W, KI, MO) \
+    if (rounding) FREP_IV_LAUNCH(1, W, KI, MO); \
+    else FREP_IV_LAUNCH(0, W, KI, MO)
+#define FREP_IV_CELLS(W, MO)                                       \
+    if ((interval_ki ? interval_ki : plan.interval_ki) == 2) {     \
+        FREP_IV_ROUND(W, 2, MO);                                   \
+    } else {                                                       \
+        FREP_IV_ROUND(W, 1, MO);                                   \
     }
+    if (rounding == 2) {
+        if (w == 4) FREP_IV_LAUNCH(2, 4, 1, false);
+        else FREP_IV_LAUNCH(2, 1, 1, false);
+    } else if (plan.micro && a.level == 0) {  // (the root level)
+        if (w == 4) {
+            FREP_IV_CELLS(4, true)
+        } else {
+            FREP_IV_CELLS(1, true)
+        }
+    } else if (w == 4) {
+        FREP_IV_CELLS(4, false)
+    } else {
+        FREP_IV_CELLS(1, false)
+    }
+#undef FREP_IV_CELLS
+#undef FREP_IV_ROUND
 #undef FREP_IV_LAUNCH
     return cudaGetLastError();
 }
