@@ -196,7 +196,9 @@ struct RenderArgs {
                                      //   reference's layout, offsets from hdr
 };
 
-cudaError_t launch_render(const RenderArgs& a, cudaStream_t stream);
+// `layers` > 1: that many jittered frames into consecutive images (rgba8 and
+// hits hold `layers` times width x height), jitter seeds jitter_seed + 0, 1, ...
+cudaError_t launch_render(const RenderArgs& a, cudaStream_t stream, uint32_t layers = 1);
 // out[p] = rounded mean of the n layers' rgb at pixel p, alpha 255 (layers:
 // n consecutive rgba8 images of `pixels` pixels).
 cudaError_t launch_resolve_layers(const uint8_t* layers, uint32_t n, uint32_t pixels, uint8_t* out,

@@ -9,26 +9,47 @@
 // Blocks are 8 x 8 pixel tiles, so that neighbouring rays (which walk the same
 // nodes and usually share the hit node's tape) sit in the same warp.
 #include <algorithm>
+#include "cell_div.h"
 #include "device_common.cuh"
 #include "kernels.h"
 
 namespace frep {
 namespace dev {
 
+constexpr uint32_t RENDER_THREADS = 64;
+
 struct RHit {
     float t;
     uint32_t node, level, cell, steps;
 };
 
-struct Tree {
+// What a step needs of a level, in a warp's shared memory (two 16-byte reads
+// where a ray changes its level): the address of the level's first record and
+// the bytes of one, the words of a mask, the cells along an axis, the cell size
+// and its reciprocal, and the largest distance that div_by takes (0: none).
+struct __align__(16) Level {
     const uint32_t* nodes;
-    const RenderArgs* a;
-    unsigned long long ofs[MAX_LEVELS];
-
-    __device__ const uint32_t* rec(uint32_t lvl, uint32_t node) const {
-        return nodes + ofs[lvl] + (size_t)node * a->node_size[lvl];
-    }
+    uint32_t size, words;
+    float dim, cell, rcell, vmax;
 };
+
+template <bool CMP>
+__device__ __forceinline__ void load_levels(const RenderArgs& A, Level* lv) {
+    const uint32_t l = threadIdx.x & 31;
+    if (l < A.levels) {
+        const unsigned long long ofs = CMP ? A.node_ofs[l] : __ldg(&A.hdr->node_ofs[l]);
+        const uint32_t dim = A.dims[l];
+        const float cs = A.cell_size[l];
+        lv[l] = Level{A.nodes + ofs, A.node_size[l] * 4, dim * dim * dim >> 5, (float)dim, cs, __frcp_rn(cs),
+                      cs >= DIV_BY_DMIN && cs <= DIV_BY_DMAX ? DIV_BY_MAX : 0.0f};
+    }
+    __syncwarp();
+}
+
+__device__ __forceinline__ const uint32_t* node_rec(const Level& l, uint32_t node) {
+    return reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(l.nodes) +
+                                             (unsigned long long)node * l.size);
+}
 
 // Where a node record keeps its masks and children. CMP = false: the
 // reference's layout (node.comp:4-72), [tape, coords, leaf, interior,
@@ -40,24 +61,26 @@ template <bool CMP>
 struct Layout;
 template <>
 struct Layout<false> {
-    static __device__ __forceinline__ bool leaf(const uint32_t* r, uint32_t c3, uint32_t idx) {
-        return (__ldg(&r[4 + (idx >> 5)]) >> (idx & 31)) & 1u;
+    static __device__ __forceinline__ uint32_t leaf_word(const uint32_t* r, uint32_t W, uint32_t idx) {
+        return __ldg(&r[4 + (idx >> 5)]);
     }
-    // The child node of an interior cell, or ~0 when the cell is not interior.
-    static __device__ __forceinline__ uint32_t child(const uint32_t* r, uint32_t c3, uint32_t idx) {
-        if (!((__ldg(&r[4 + c3 / 32 + (idx >> 5)]) >> (idx & 31)) & 1u)) return ~0u;
-        return __ldg(&r[4 + c3 / 16 + idx]);
+    static __device__ __forceinline__ uint32_t interior_word(const uint32_t* r, uint32_t W, uint32_t idx) {
+        return __ldg(&r[4 + W + (idx >> 5)]);
+    }
+    // The child node of an interior cell, whose interior word is iw.
+    static __device__ __forceinline__ uint32_t child(const uint32_t* r, uint32_t W, uint32_t idx, uint32_t iw) {
+        return __ldg(&r[4 + 2 * W + idx]);
     }
 };
 template <>
 struct Layout<true> {
-    static __device__ __forceinline__ bool leaf(const uint32_t* r, uint32_t c3, uint32_t idx) {
-        return (__ldg(&r[1 + (idx >> 5)]) >> (idx & 31)) & 1u;
+    static __device__ __forceinline__ uint32_t leaf_word(const uint32_t* r, uint32_t W, uint32_t idx) {
+        return __ldg(&r[1 + (idx >> 5)]);
     }
-    static __device__ __forceinline__ uint32_t child(const uint32_t* r, uint32_t c3, uint32_t idx) {
-        const uint32_t W = c3 >> 5;
-        const uint32_t iw = __ldg(&r[1 + W + (idx >> 5)]);
-        if (!((iw >> (idx & 31)) & 1u)) return ~0u;
+    static __device__ __forceinline__ uint32_t interior_word(const uint32_t* r, uint32_t W, uint32_t idx) {
+        return __ldg(&r[1 + W + (idx >> 5)]);
+    }
+    static __device__ __forceinline__ uint32_t child(const uint32_t* r, uint32_t W, uint32_t idx, uint32_t iw) {
         return __ldg(&r[1 + 3 * W]) + __ldg(&r[1 + 2 * W + (idx >> 5)]) + __popc(iw & ((1u << (idx & 31)) - 1u));
     }
 };
@@ -79,136 +102,280 @@ __device__ bool grid_intersect(const RenderArgs& A, float3 o, float3 inv, float&
     return te <= tl && tl >= 0.0f;
 }
 
+// A ray and where it enters and leaves the grid.
+struct Ray {
+    float3 o, d, inv;
+    float enter, leave;
+};
+__device__ __forceinline__ bool ray_setup(const RenderArgs& A, float3 o, float3 d, Ray& ray) {
+    ray.o = o;
+    ray.d = d;
+    ray.inv = make_float3(__fdiv_rn(1.0f, d.x), __fdiv_rn(1.0f, d.y), __fdiv_rn(1.0f, d.z));
+    return grid_intersect(A, o, ray.inv, ray.enter, ray.leave);
+}
+
 // dda (main.comp:46-111), kd-restart. Cell coordinates are clamped to
 // [0, dim) and the step count is bounded (both also in the oracle).
+//
+// Bound by issue and by the length of the chain of one step (a twentieth of a
+// frame's warps, those along the surface, take most of its time): the
+// reference's two nested loops (walk down, restart at the root) are one, so
+// that every trip is one step of every live ray (nested, a lane that restarts
+// waits for all lanes of its warp to leave the inner loop); restart and descent
+// share the code that enters a level; cell numbers are computed in floats, by
+// a sum rounded down at 2^23, without conversions; the divisions by the cell
+// size are five operations each with its reciprocal (div_by) instead of a
+// general division; the leaf and interior words are read together (the child
+// number with them as well was slower, 0.55 against 0.52 ms: more lines).
+// 2048^3 scene at 1080p 1.20 -> 0.52 ms, 128 frames of 512^2 6.2 -> 3.2 ms, a
+// ray that runs into the step bound 18 to 54 -> 11 to 16 ms.
 template <bool CMP>
-__device__ bool dda(const Tree& T, float3 o, float3 d, RHit& hit) {
-    const RenderArgs& A = *T.a;
-    hit.steps = 0;
-    const float3 inv = make_float3(__fdiv_rn(1.0f, d.x), __fdiv_rn(1.0f, d.y), __fdiv_rn(1.0f, d.z));
-    float g_enter, g_leave;
-    if (!grid_intersect(A, o, inv, g_enter, g_leave)) return false;
+__device__ bool dda(const RenderArgs& A, const Level* lv, const Ray& ray, RHit& hit) {
+    constexpr float MAGIC = 0x1p23f;
+    const float3 o = ray.o, d = ray.d, inv = ray.inv;
     const float sx = inv.x >= 0.0f ? 1.0f : 0.0f, sy = inv.y >= 0.0f ? 1.0f : 0.0f,
                 sz = inv.z >= 0.0f ? 1.0f : 0.0f;
-    float t_curr = __fadd_rn(max_sel(g_enter, 0.0f), EPS);
-    float t_max = t_curr;
-    uint32_t steps = 0;
     const uint32_t last = A.levels - 1;
-    while (t_max < __fsub_rn(g_leave, EPS)) {
-        uint32_t lvl = 0, node = 0;
-        float npx = A.low[0], npy = A.low[1], npz = A.low[2];
-        t_curr = __fadd_rn(t_max, EPS);
-        t_max = g_leave;
-        while (t_curr < __fsub_rn(t_max, EPS)) {
-            if (++steps > MAX_DDA_STEPS) { hit.steps = steps; return false; }
-            const float cs = A.cell_size[lvl];
-            const int dim = (int)A.dims[lvl];
-            const float te = __fadd_rn(t_curr, EPS);
-            const float nx = __fdiv_rn(__fsub_rn(__fadd_rn(o.x, __fmul_rn(te, d.x)), npx), cs);
-            const float ny = __fdiv_rn(__fsub_rn(__fadd_rn(o.y, __fmul_rn(te, d.y)), npy), cs);
-            const float nz = __fdiv_rn(__fsub_rn(__fadd_rn(o.z, __fmul_rn(te, d.z)), npz), cs);
-            int cx = (int)floorf(nx), cy = (int)floorf(ny), cz = (int)floorf(nz);
-            cx = min(max(cx, 0), dim - 1);
-            cy = min(max(cy, 0), dim - 1);
-            cz = min(max(cz, 0), dim - 1);
-            const float tnx = __fadd_rn(te, __fmul_rn(__fmul_rn(__fsub_rn(__fadd_rn((float)cx, sx), nx), cs), inv.x));
-            const float tny = __fadd_rn(te, __fmul_rn(__fmul_rn(__fsub_rn(__fadd_rn((float)cy, sy), ny), cs), inv.y));
-            const float tnz = __fadd_rn(te, __fmul_rn(__fmul_rn(__fsub_rn(__fadd_rn((float)cz, sz), nz), cs), inv.z));
-            const uint32_t idx = (uint32_t)(cz + dim * cy + dim * dim * cx);
-            const uint32_t* r = T.rec(lvl, node);
-            const uint32_t c3 = (uint32_t)(dim * dim * dim);
-            if (Layout<CMP>::leaf(r, c3, idx)) {
-                hit.t = t_curr;
-                hit.node = node;
-                hit.level = lvl;
-                hit.cell = idx;
-                hit.steps = steps;
-                return true;
+    const float g_leave = ray.leave, g_stop = __fsub_rn(g_leave, EPS);
+    // No step before the first restart: t_curr < t_max - EPS does not hold.
+    float t_max = __fadd_rn(max_sel(ray.enter, 0.0f), EPS), t_curr = t_max;
+    uint32_t steps = 0, lvl = 0, node = 0, W = 0;
+    float cs = 1.0f, rcs = 1.0f, vmax = 0.0f, fdim = 0.0f, npx = 0.0f, npy = 0.0f, npz = 0.0f;
+    const uint32_t* r = nullptr;
+    bool entered = false;
+    while (true) {
+        if (!(t_curr < __fsub_rn(t_max, EPS))) {  // the node is left: restart at the root
+            if (!(t_max < g_stop)) break;
+            t_curr = __fadd_rn(t_max, EPS);
+            t_max = g_leave;
+            if (!(t_curr < g_stop)) break;
+            lvl = 0;
+            node = 0;
+            npx = A.low[0];
+            npy = A.low[1];
+            npz = A.low[2];
+            entered = true;
+        }
+        if (entered) {
+            const Level l = lv[lvl];
+            r = node_rec(l, node);
+            cs = l.cell;
+            rcs = l.rcell;
+            vmax = l.vmax;
+            fdim = l.dim;
+            W = l.words;
+        }
+        if (++steps > MAX_DDA_STEPS) break;
+        const float te = __fadd_rn(t_curr, EPS);
+        const float vx = __fsub_rn(__fadd_rn(o.x, __fmul_rn(te, d.x)), npx);
+        const float vy = __fsub_rn(__fadd_rn(o.y, __fmul_rn(te, d.y)), npy);
+        const float vz = __fsub_rn(__fadd_rn(o.z, __fmul_rn(te, d.z)), npz);
+        float nx = div_by(vx, cs, rcs), ny = div_by(vy, cs, rcs), nz = div_by(vz, cs, rcs);
+        if (!(fminf(fminf(fabsf(vx), fabsf(vy)), fabsf(vz)) >= DIV_BY_MIN &&
+              fmaxf(fmaxf(fabsf(vx), fabsf(vy)), fabsf(vz)) <= vmax)) {
+            // Outside the range, but for zeros, whose sign alone may differ:
+            // it reaches no result below.
+            const auto fits = [&](float v) { return v == 0.0f ? vmax > 0.0f : fabsf(v) >= DIV_BY_MIN && fabsf(v) <= vmax; };
+            if (!(fits(vx) && fits(vy) && fits(vz))) {
+                nx = __fdiv_rn(vx, cs);
+                ny = __fdiv_rn(vy, cs);
+                nz = __fdiv_rn(vz, cs);
             }
-            const uint32_t ch = lvl < last ? Layout<CMP>::child(r, c3, idx) : ~0u;
-            if (ch != ~0u) {
-                node = ch;
-                npx = __fadd_rn(npx, __fmul_rn((float)cx, cs));
-                npy = __fadd_rn(npy, __fmul_rn((float)cy, cs));
-                npz = __fadd_rn(npz, __fmul_rn((float)cz, cs));
-                t_max = min_sel(tnx, min_sel(tny, tnz));
-                lvl++;
-            } else {
-                t_curr = min_sel(tnx, min_sel(tny, tnz));
-            }
+        }
+        // floor and clamp to [0, dim): clamped first (a NaN gives 0), then
+        // MAGIC + v rounded down is MAGIC + floor(v).
+        const float top = __fsub_rn(fdim, 1.0f);
+        const float cx = __fsub_rn(__fadd_rd(fminf(fmaxf(nx, 0.0f), top), MAGIC), MAGIC);
+        const float cy = __fsub_rn(__fadd_rd(fminf(fmaxf(ny, 0.0f), top), MAGIC), MAGIC);
+        const float uz = __fadd_rd(fminf(fmaxf(nz, 0.0f), top), MAGIC), cz = __fsub_rn(uz, MAGIC);
+        // z + dim y + dim^2 x < 2^15: exact, in the low bits beside MAGIC.
+        const uint32_t idx = __float_as_uint(__fmaf_rn(__fmaf_rn(cx, fdim, cy), fdim, uz)) & 0x7FFFFFu;
+        const uint32_t leaf = Layout<CMP>::leaf_word(r, W, idx);
+        const uint32_t inner = lvl < last ? Layout<CMP>::interior_word(r, W, idx) : 0u;
+        const float tnx = __fadd_rn(te, __fmul_rn(__fmul_rn(__fsub_rn(__fadd_rn(cx, sx), nx), cs), inv.x));
+        const float tny = __fadd_rn(te, __fmul_rn(__fmul_rn(__fsub_rn(__fadd_rn(cy, sy), ny), cs), inv.y));
+        const float tnz = __fadd_rn(te, __fmul_rn(__fmul_rn(__fsub_rn(__fadd_rn(cz, sz), nz), cs), inv.z));
+        const float tn = min_sel(tnx, min_sel(tny, tnz));
+        if ((leaf >> (idx & 31)) & 1u) {
+            hit.t = t_curr;
+            hit.node = node;
+            hit.level = lvl;
+            hit.cell = idx;
+            hit.steps = steps;
+            return true;
+        }
+        entered = (inner >> (idx & 31)) & 1u;
+        if (entered) {
+            node = Layout<CMP>::child(r, W, idx, inner);
+            lvl++;
+            npx = __fadd_rn(npx, __fmul_rn(cx, cs));
+            npy = __fadd_rn(npy, __fmul_rn(cy, cs));
+            npz = __fadd_rn(npz, __fmul_rn(cz, cs));
+            t_max = tn;
+        } else {
+            t_curr = tn;
         }
     }
     hit.steps = steps;
     return false;
 }
 
+// The gradient of the operations that the common path leaves out.
+__device__ __noinline__ float4 gradient_rare(uint32_t op, float4 a, float4 b) {
+    switch (op) {
+        case OP_SIN: {
+            const float c = frep_cosf(a.w);
+            return make_float4(__fmul_rn(c, a.x), __fmul_rn(c, a.y), __fmul_rn(c, a.z), frep_sinf(a.w));
+        }
+        case OP_COS: {
+            const float ms = -frep_sinf(a.w);
+            return make_float4(__fmul_rn(ms, a.x), __fmul_rn(ms, a.y), __fmul_rn(ms, a.z), frep_cosf(a.w));
+        }
+        case OP_DIV: {
+            const float dd = __fmul_rn(b.w, b.w);
+            return make_float4(__fdiv_rn(__fsub_rn(__fmul_rn(a.x, b.w), __fmul_rn(a.w, b.x)), dd),
+                               __fdiv_rn(__fsub_rn(__fmul_rn(a.y, b.w), __fmul_rn(a.w, b.y)), dd),
+                               __fdiv_rn(__fsub_rn(__fmul_rn(a.z, b.w), __fmul_rn(a.w, b.z)), dd),
+                               __fdiv_rn(a.w, b.w));
+        }
+        case OP_EXP: {
+            const float e = frep_expf(a.w);
+            return make_float4(__fmul_rn(e, a.x), __fmul_rn(e, a.y), __fmul_rn(e, a.z), e);
+        }
+        default: {  // SQRT
+            const float sq = __fsqrt_rn(a.w);
+            const float dd = __fmul_rn(2.0f, sq);
+            return make_float4(__fdiv_rn(a.x, dd), __fdiv_rn(a.y, dd), __fdiv_rn(a.z, dd), sq);
+        }
+    }
+}
+
+__device__ __forceinline__ float flip(float v, uint32_t sign) { return __uint_as_float(__float_as_uint(v) ^ sign); }
+
 // tape_eval_gradient (gradient.comp:4-88) with a per-thread slot array of NS
-// entries (local memory).
+// entries (local memory; in shared memory the slots cost the walk its L1:
+// 0.72 against 0.63 ms for the 2048^3 scene at 1080p). The lanes run the tapes
+// of different nodes, so a switch over the operation runs most of its arms on
+// each trip, each behind the dispatch: the common operations are computed
+// together and selected, and the next word is on its way while one runs.
 template <int NS>
 __device__ float3 gradient(const uint64_t* tape, uint32_t n, float x, float y, float z, float t) {
+    constexpr uint32_t RARE = 1u << OP_SIN | 1u << OP_COS | 1u << OP_DIV | 1u << OP_EXP | 1u << OP_SQRT;
     float4 s[NS];
     s[0] = make_float4(1, 0, 0, x);
     s[1] = make_float4(0, 1, 0, y);
     s[2] = make_float4(0, 0, 1, z);
     s[3] = make_float4(0, 0, 0, t);
+    uint64_t next = n ? __ldg(&tape[0]) : 0;
     for (uint32_t i = 0; i < n; i++) {
-        const uint64_t w = __ldg(&tape[i]);
+        const uint64_t w = next;
+        if (i + 1 < n) next = __ldg(&tape[i + 1]);
         const uint32_t op = w_op(w);
+        const float4 a = s[op == OP_CONST ? 0u : w_a(w)], b = s[is_binary(op) ? w_b(w) : 0u];
         float4 r;
-        if (op == OP_CONST) {
-            r = make_float4(0, 0, 0, w_const(w));
+        if ((RARE >> op) & 1u) {
+            r = gradient_rare(op, a, b);
         } else {
-            const float4 a = s[w_a(w)], b = s[w_b(w)];
-            switch (op) {
-                case OP_SIN: {
-                    const float c = frep_cosf(a.w);
-                    r = make_float4(__fmul_rn(c, a.x), __fmul_rn(c, a.y), __fmul_rn(c, a.z), frep_sinf(a.w));
-                    break;
-                }
-                case OP_COS: {
-                    const float ms = -frep_sinf(a.w);
-                    r = make_float4(__fmul_rn(ms, a.x), __fmul_rn(ms, a.y), __fmul_rn(ms, a.z), frep_cosf(a.w));
-                    break;
-                }
-                case OP_ADD:
-                    r = make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
-                    break;
-                case OP_SUB:
-                    r = make_float4(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y), __fsub_rn(a.z, b.z), __fsub_rn(a.w, b.w));
-                    break;
-                case OP_MUL:
-                    r = make_float4(__fadd_rn(__fmul_rn(a.x, b.w), __fmul_rn(a.w, b.x)),
-                                    __fadd_rn(__fmul_rn(a.y, b.w), __fmul_rn(a.w, b.y)),
-                                    __fadd_rn(__fmul_rn(a.z, b.w), __fmul_rn(a.w, b.z)), __fmul_rn(a.w, b.w));
-                    break;
-                case OP_DIV: {
-                    const float dd = __fmul_rn(b.w, b.w);
-                    r = make_float4(__fdiv_rn(__fsub_rn(__fmul_rn(a.x, b.w), __fmul_rn(a.w, b.x)), dd),
-                                    __fdiv_rn(__fsub_rn(__fmul_rn(a.y, b.w), __fmul_rn(a.w, b.y)), dd),
-                                    __fdiv_rn(__fsub_rn(__fmul_rn(a.z, b.w), __fmul_rn(a.w, b.z)), dd),
-                                    __fdiv_rn(a.w, b.w));
-                    break;
-                }
-                case OP_MIN: r = (a.w < b.w) ? a : b; break;
-                case OP_MAX: r = (a.w > b.w) ? a : b; break;
-                case OP_EXP: {
-                    const float e = frep_expf(a.w);
-                    r = make_float4(__fmul_rn(e, a.x), __fmul_rn(e, a.y), __fmul_rn(e, a.z), e);
-                    break;
-                }
-                case OP_NEG: r = make_float4(-a.x, -a.y, -a.z, -a.w); break;
-                case OP_SQRT: {
-                    const float sq = __fsqrt_rn(a.w);
-                    const float dd = __fmul_rn(2.0f, sq);
-                    r = make_float4(__fdiv_rn(a.x, dd), __fdiv_rn(a.y, dd), __fdiv_rn(a.z, dd), sq);
-                    break;
-                }
-                default: r = a; break;  // COPY
+            // ADD, SUB (a + -b), MUL (the product rule), and for the others
+            // one operand, its sign flipped for NEG.
+            const uint32_t sub = op == OP_SUB ? 0x80000000u : 0u, neg = op == OP_NEG ? 0x80000000u : 0u;
+            const bool second = (op == OP_MIN && !(a.w < b.w)) || (op == OP_MAX && !(a.w > b.w));
+            const bool mul = op == OP_MUL;
+            r.x = mul ? __fadd_rn(__fmul_rn(a.x, b.w), __fmul_rn(a.w, b.x)) : flip(second ? b.x : a.x, neg);
+            r.y = mul ? __fadd_rn(__fmul_rn(a.y, b.w), __fmul_rn(a.w, b.y)) : flip(second ? b.y : a.y, neg);
+            r.z = mul ? __fadd_rn(__fmul_rn(a.z, b.w), __fmul_rn(a.w, b.z)) : flip(second ? b.z : a.z, neg);
+            r.w = mul ? __fmul_rn(a.w, b.w) : flip(second ? b.w : a.w, neg);
+            if (op == OP_ADD || op == OP_SUB) {
+                r.x = __fadd_rn(a.x, flip(b.x, sub));
+                r.y = __fadd_rn(a.y, flip(b.y, sub));
+                r.z = __fadd_rn(a.z, flip(b.z, sub));
+                r.w = __fadd_rn(a.w, flip(b.w, sub));
             }
+            if (op == OP_CONST) r = make_float4(0, 0, 0, w_const(w));
         }
         s[w_out(w)] = r;
     }
     return make_float3(s[0].x, s[0].y, s[0].z);
+}
+
+// The same for one tape that all 32 lanes run (each at its own point): the
+// lanes decode 32 words at once into `stage` (a warp's 32 records in shared
+// memory), and every branch is the warp's.
+template <int NS>
+__device__ float3 gradient_shared_tape(const uint64_t* tape, uint32_t n, float x, float y, float z, float t,
+                                       uint4* stage) {
+    const uint32_t lane = threadIdx.x & 31;
+    float4 s[NS];
+    s[0] = make_float4(1, 0, 0, x);
+    s[1] = make_float4(0, 1, 0, y);
+    s[2] = make_float4(0, 0, 1, z);
+    s[3] = make_float4(0, 0, 0, t);
+    uint64_t next = lane < n ? __ldg(&tape[lane]) : 0;
+    for (uint32_t base = 0; base < n; base += 32) {
+        const uint64_t w = next;
+        if (base + 32 + lane < n) next = __ldg(&tape[base + 32 + lane]);
+        const uint32_t op = w_op(w);
+        __syncwarp();
+        stage[lane] = make_uint4(op == OP_CONST ? (uint32_t)(w >> 32) : w_a(w), is_binary(op) ? w_b(w) : 0u, w_out(w), op);
+        __syncwarp();
+        const uint32_t m = min(n - base, 32u);
+        uint4 rec = stage[0];
+        for (uint32_t j = 0; j < m; j++) {
+            const uint4 q = rec;
+            rec = stage[(j + 1) & 31];
+            float4 r;
+            if (q.w == OP_CONST) {
+                r = make_float4(0, 0, 0, __uint_as_float(q.x));
+            } else {
+                const float4 a = s[q.x], b = s[q.y];
+                if (q.w == OP_MUL)
+                    r = make_float4(__fadd_rn(__fmul_rn(a.x, b.w), __fmul_rn(a.w, b.x)),
+                                    __fadd_rn(__fmul_rn(a.y, b.w), __fmul_rn(a.w, b.y)),
+                                    __fadd_rn(__fmul_rn(a.z, b.w), __fmul_rn(a.w, b.z)), __fmul_rn(a.w, b.w));
+                else if (q.w == OP_ADD)
+                    r = make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
+                else if (q.w == OP_SUB)
+                    r = make_float4(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y), __fsub_rn(a.z, b.z), __fsub_rn(a.w, b.w));
+                else if (is_mm(q.w))
+                    r = (q.w == OP_MIN ? a.w < b.w : a.w > b.w) ? a : b;
+                else if (q.w == OP_NEG)
+                    r = make_float4(-a.x, -a.y, -a.z, -a.w);
+                else if (q.w == OP_COPY)
+                    r = a;
+                else
+                    r = gradient_rare(q.w, a, b);
+            }
+            s[q.z] = r;
+        }
+    }
+    return make_float3(s[0].x, s[0].y, s[0].z);
+}
+
+// The normals' gradients of a warp: lanes with `need` set have a tape of n
+// words. A tape much longer than the others' (a hit on a full cell of the root
+// has the whole shape's) runs first, for its lanes alone: in lockstep a word
+// costs about 250 cycles, on its own 140 (a warp by itself), so it is taken out
+// when the rest then has at most half its trips; a warp with one tape always.
+// (A 25,000-word root tape: 3.3 -> 1.8 ms of one warp. Taking every tape out
+// that is the longest: 0.65 against 0.59 ms for the 2048^3 scene.)
+template <int NS>
+__device__ float3 warp_gradient(bool need, const uint64_t* tape, uint32_t n, float3 p, float t, uint4* stage) {
+    float3 g = make_float3(0.0f, 0.0f, 0.0f);
+    while (true) {
+        const uint32_t longest = __reduce_max_sync(~0u, need ? n : 0u);
+        if (longest == 0) break;
+        const int lead = __ffs(__ballot_sync(~0u, need && n == longest)) - 1;
+        const unsigned long long lt = __shfl_sync(~0u, reinterpret_cast<unsigned long long>(tape), lead);
+        const bool mine = need && reinterpret_cast<unsigned long long>(tape) == lt;
+        if (__reduce_max_sync(~0u, need && !mine ? n : 0u) > longest / 2) break;
+        const float3 v = gradient_shared_tape<NS>(reinterpret_cast<const uint64_t*>(lt), longest, p.x, p.y, p.z, t, stage);
+        if (mine) {
+            g = v;
+            need = false;
+        }
+    }
+    if (need) g = gradient<NS>(tape, n, p.x, p.y, p.z, t);
+    return g;
 }
 
 __device__ __forceinline__ float dot3(float3 a, float3 b) {
@@ -240,16 +407,17 @@ struct HitRecord {  // == frep_hit
 };
 
 template <int NS, bool CMP>
-__device__ __forceinline__ void render_pixel(const RenderArgs& A, uint32_t x, uint32_t y) {
-    Tree T;
-    T.nodes = A.nodes;
-    T.a = &A;
-    for (uint32_t l = 0; l < A.levels; l++) T.ofs[l] = CMP ? A.node_ofs[l] : A.hdr->node_ofs[l];
+__device__ __forceinline__ void render_pixel(const RenderArgs& A, uint32_t x, uint32_t y, uint32_t layer) {
+    __shared__ uint4 stage[RENDER_THREADS];
+    __shared__ Level levels[RENDER_THREADS / 32][MAX_LEVELS];
+    Level* const lv = levels[threadIdx.x >> 5];
+    // Lanes past the image's edge stay for the warp's joint work.
+    const bool inside = x < A.width && y < A.height;
 
     // Ray generation (main.comp:168-178).
     float ox = 0.0f, oy = 0.0f;
     if (A.jitter) {
-        float seed = A.jitter_seed;
+        float seed = __fadd_rn(A.jitter_seed, (float)layer);
         const float r0 = rand_step(seed, x, y);
         const float r1 = rand_step(seed, x, y);
         ox = __fmul_rn(2.0f, __fsub_rn(r0, 0.5f));
@@ -273,7 +441,30 @@ __device__ __forceinline__ void render_pixel(const RenderArgs& A, uint32_t x, ui
     }
 
     RHit h;
-    const bool did = dda<CMP>(T, o, d, h);
+    h.t = 0.0f;
+    h.steps = 0;
+    Ray ray;
+    bool did = inside && ray_setup(A, o, d, ray);
+    if (__ballot_sync(~0u, did)) {
+        load_levels<CMP>(A, lv);
+        did = did && dda<CMP>(A, lv, ray, h);
+    }
+    const bool lit = did && !(h.t < 0.0f);
+    const float px = __fadd_rn(o.x, __fmul_rn(h.t, d.x));
+    const float py = __fadd_rn(o.y, __fmul_rn(h.t, d.y));
+    const float pz = __fadd_rn(o.z, __fmul_rn(h.t, d.z));
+    float3 grad = make_float3(0.0f, 0.0f, 0.0f);
+    if (__ballot_sync(~0u, lit)) {
+        const uint64_t* tape = nullptr;
+        uint32_t tn = 0;
+        if (lit) {
+            const uint32_t tidx = __ldg(&node_rec(lv[h.level], h.node)[0]);
+            tn = (uint32_t)__ldg(&A.tapes[tidx]);
+            tape = A.tapes + tidx + 1;
+        }
+        grad = warp_gradient<NS>(lit, tape, tn, make_float3(px, py, pz), A.tape_time, stage + (threadIdx.x & ~31u));
+    }
+    if (!inside) return;
     float col[4];
     float3 n = make_float3(0.0f, 0.0f, 0.0f);
     if (!did) {
@@ -281,12 +472,7 @@ __device__ __forceinline__ void render_pixel(const RenderArgs& A, uint32_t x, ui
     } else if (h.t < 0.0f) {  // main.comp:149-151
         for (int c = 0; c < 4; c++) col[c] = 1.0f;
     } else {  // shade (main.comp:115-139)
-        const uint32_t tidx = __ldg(&T.rec(h.level, h.node)[0]);
-        const uint32_t tn = (uint32_t)__ldg(&A.tapes[tidx]);
-        const float px = __fadd_rn(o.x, __fmul_rn(h.t, d.x));
-        const float py = __fadd_rn(o.y, __fmul_rn(h.t, d.y));
-        const float pz = __fadd_rn(o.z, __fmul_rn(h.t, d.z));
-        n = normalize3(gradient<NS>(A.tapes + tidx + 1, tn, px, py, pz, A.tape_time));
+        n = normalize3(grad);
         float diff[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         for (uint32_t i = 0; i < A.n_lights; i++) {
             const float3 L = make_float3(A.light_dir[i][0], A.light_dir[i][1], A.light_dir[i][2]);
@@ -295,7 +481,8 @@ __device__ __forceinline__ void render_pixel(const RenderArgs& A, uint32_t x, ui
                 const float3 so = make_float3(__fadd_rn(o.x, __fmul_rn(ts, d.x)), __fadd_rn(o.y, __fmul_rn(ts, d.y)),
                                               __fadd_rn(o.z, __fmul_rn(ts, d.z)));
                 RHit sh;
-                if (dda<CMP>(T, so, make_float3(-L.x, -L.y, -L.z), sh)) continue;
+                Ray sr;
+                if (ray_setup(A, so, make_float3(-L.x, -L.y, -L.z), sr) && dda<CMP>(A, lv, sr, sh)) continue;
             }
             const float dd = dot3(make_float3(-L.x, -L.y, -L.z), n);
             const float inten = fmaxf(dd, 0.0f);
@@ -303,7 +490,7 @@ __device__ __forceinline__ void render_pixel(const RenderArgs& A, uint32_t x, ui
         }
         for (int c = 0; c < 4; c++) col[c] = __fadd_rn(A.ambient[c], diff[c]);
     }
-    const size_t pix = (size_t)y * A.width + x;
+    const size_t pix = ((size_t)layer * A.height + y) * A.width + x;
     if (A.rgba8) {
         uchar4 v = make_uchar4(to_unorm8(col[0]), to_unorm8(col[1]), to_unorm8(col[2]), to_unorm8(col[3]));
         reinterpret_cast<uchar4*>(A.rgba8)[pix] = v;
@@ -322,22 +509,22 @@ __device__ __forceinline__ void render_pixel(const RenderArgs& A, uint32_t x, ui
     }
 }
 
+// blockIdx.z: the layer of a multi-sample image (jitter seeds one apart), whose
+// layers follow one another in the outputs.
 template <int NS, bool CMP = false>
-__global__ void __launch_bounds__(64) render_kernel(const RenderArgs A) {
+__global__ void __launch_bounds__(RENDER_THREADS) render_kernel(const RenderArgs A, uint32_t layer0) {
     const uint32_t x = blockIdx.x * 8 + (threadIdx.x & 7);
     const uint32_t y = blockIdx.y * 8 + (threadIdx.x >> 3);
-    if (x >= A.width || y >= A.height) return;
-    render_pixel<NS, CMP>(A, x, y);
+    render_pixel<NS, CMP>(A, x, y, layer0 + blockIdx.z);
 }
 
 // Many frames in one launch: blockIdx.z selects the frame.
 template <int NS>
-__global__ void __launch_bounds__(64) render_batch_kernel(const RenderArgs* args) {
+__global__ void __launch_bounds__(RENDER_THREADS) render_batch_kernel(const RenderArgs* args) {
     const RenderArgs& A = args[blockIdx.z];
     const uint32_t x = blockIdx.x * 8 + (threadIdx.x & 7);
     const uint32_t y = blockIdx.y * 8 + (threadIdx.x >> 3);
-    if (x >= A.width || y >= A.height) return;
-    render_pixel<NS, false>(A, x, y);
+    render_pixel<NS, false>(A, x, y, 0);
 }
 
 // Temporal resolve (renderer/triangle.frag:14-23): the pixel is the mean of
@@ -371,41 +558,43 @@ cudaError_t launch_resolve_layers(const uint8_t* layers, uint32_t n, uint32_t pi
     return cudaGetLastError();
 }
 
-cudaError_t launch_render(const RenderArgs& a, cudaStream_t stream) {
-    const dim3 grid((a.width + 7) / 8, (a.height + 7) / 8);
+template <bool CMP>
+static void render_launch(const RenderArgs& a, dim3 grid, uint32_t layer0, cudaStream_t stream) {
+    constexpr uint32_t T = dev::RENDER_THREADS;
     const uint32_t ns = a.n_slots;
-    if (a.compact) {
-        if (ns <= 32) dev::render_kernel<32, true><<<grid, 64, 0, stream>>>(a);
-        else if (ns <= 64) dev::render_kernel<64, true><<<grid, 64, 0, stream>>>(a);
-        else if (ns <= 128) dev::render_kernel<128, true><<<grid, 64, 0, stream>>>(a);
-        else if (ns <= 256) dev::render_kernel<256, true><<<grid, 64, 0, stream>>>(a);
-        else if (ns <= 512) dev::render_kernel<512, true><<<grid, 64, 0, stream>>>(a);
-        else if (ns <= 1024) dev::render_kernel<1024, true><<<grid, 64, 0, stream>>>(a);
-        else return cudaErrorInvalidValue;
-        return cudaGetLastError();
+    if (ns <= 32) dev::render_kernel<32, CMP><<<grid, T, 0, stream>>>(a, layer0);
+    else if (ns <= 64) dev::render_kernel<64, CMP><<<grid, T, 0, stream>>>(a, layer0);
+    else if (ns <= 128) dev::render_kernel<128, CMP><<<grid, T, 0, stream>>>(a, layer0);
+    else if (ns <= 256) dev::render_kernel<256, CMP><<<grid, T, 0, stream>>>(a, layer0);
+    else if (ns <= 512) dev::render_kernel<512, CMP><<<grid, T, 0, stream>>>(a, layer0);
+    else dev::render_kernel<1024, CMP><<<grid, T, 0, stream>>>(a, layer0);
+}
+
+cudaError_t launch_render(const RenderArgs& a, cudaStream_t stream, uint32_t layers) {
+    if (a.n_slots > 1024) return cudaErrorInvalidValue;
+    for (uint32_t at = 0; at < layers; at += 65535) {  // the largest gridDim.z
+        const dim3 grid((a.width + 7) / 8, (a.height + 7) / 8, std::min(layers - at, 65535u));
+        if (a.compact) render_launch<true>(a, grid, at, stream);
+        else render_launch<false>(a, grid, at, stream);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
     }
-    if (ns <= 32) dev::render_kernel<32><<<grid, 64, 0, stream>>>(a);
-    else if (ns <= 64) dev::render_kernel<64><<<grid, 64, 0, stream>>>(a);
-    else if (ns <= 128) dev::render_kernel<128><<<grid, 64, 0, stream>>>(a);
-    else if (ns <= 256) dev::render_kernel<256><<<grid, 64, 0, stream>>>(a);
-    else if (ns <= 512) dev::render_kernel<512><<<grid, 64, 0, stream>>>(a);
-    else if (ns <= 1024) dev::render_kernel<1024><<<grid, 64, 0, stream>>>(a);
-    else return cudaErrorInvalidValue;
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 cudaError_t launch_render_batch(const RenderArgs* args, uint32_t n, uint32_t max_w, uint32_t max_h,
                                 uint32_t max_slots, cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
-    if (n > 65535) return cudaErrorInvalidValue;
+    if (n > 65535 || max_slots > 1024) return cudaErrorInvalidValue;
+    constexpr uint32_t T = dev::RENDER_THREADS;
     const dim3 grid((max_w + 7) / 8, (max_h + 7) / 8, n);
-    if (max_slots <= 32) dev::render_batch_kernel<32><<<grid, 64, 0, stream>>>(args);
-    else if (max_slots <= 64) dev::render_batch_kernel<64><<<grid, 64, 0, stream>>>(args);
-    else if (max_slots <= 128) dev::render_batch_kernel<128><<<grid, 64, 0, stream>>>(args);
-    else if (max_slots <= 256) dev::render_batch_kernel<256><<<grid, 64, 0, stream>>>(args);
-    else if (max_slots <= 512) dev::render_batch_kernel<512><<<grid, 64, 0, stream>>>(args);
-    else if (max_slots <= 1024) dev::render_batch_kernel<1024><<<grid, 64, 0, stream>>>(args);
-    else return cudaErrorInvalidValue;
+    const uint32_t ns = max_slots;
+    if (ns <= 32) dev::render_batch_kernel<32><<<grid, T, 0, stream>>>(args);
+    else if (ns <= 64) dev::render_batch_kernel<64><<<grid, T, 0, stream>>>(args);
+    else if (ns <= 128) dev::render_batch_kernel<128><<<grid, T, 0, stream>>>(args);
+    else if (ns <= 256) dev::render_batch_kernel<256><<<grid, T, 0, stream>>>(args);
+    else if (ns <= 512) dev::render_batch_kernel<512><<<grid, T, 0, stream>>>(args);
+    else dev::render_batch_kernel<1024><<<grid, T, 0, stream>>>(args);
     return cudaGetLastError();
 }
 
