@@ -87,3 +87,17 @@ def test_temporal_layers_odd_size(ctx):
         ci = dataclasses.replace(cam, jitter=True, jitter_seed=0.5 + i)
         want, _ = orc.render(oracle.camera_vector(ci, sc.width, sc.height), rt.lights, 0.0)
         np.testing.assert_array_equal(layers[i].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("world,dims", [(2500.0, (4, 4, 4, 4)), (25000.0, (4, 4, 4)), (1e8, (4, 4))])
+def test_rays_that_stop_advancing(ctx, world, dims):
+    """Steps smaller than the spacing of t: rays repeat their cells until the
+    step bound, and their records say so."""
+    sc = scenes.random_csg(12, seed=5, grid_dims=list(dims))
+    sc = dataclasses.replace(sc, low_vertex=(-world / 2,) * 3, world_size=world)
+    vs = device_tree(ctx, sc, rounding=1)
+    orc = oracle_tree(sc, vs.tape, rounding=1)
+    d_rgba, d_hits, o_rgba, o_hits = render_both(ctx, vs, orc, sc, frep.Lights(shadow_mask=1), width=96, height=64)
+    np.testing.assert_array_equal(d_hits[..., 7], o_hits[..., 7])
+    assert o_hits[..., 7].max() == 65537
+    np.testing.assert_array_equal(d_rgba, o_rgba)
