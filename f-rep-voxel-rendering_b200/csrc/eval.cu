@@ -10,8 +10,12 @@
 // checks of the outward mode measure: every interval must contain the tape's
 // value at any point of its box.
 //
-// One thread per point or box; the slot file lives in global memory as rows
-// [slot][item] (coalesced), allocated per call.
+// One thread per box; the slot file lives in global memory as rows [slot][item]
+// (coalesced), allocated per call. Points keep their slots in shared memory
+// where a tape's slots fit (eval_points_shared_kernel).
+#include <algorithm>
+#include <vector>
+
 #include "capi_internal.h"
 
 namespace frep {
@@ -37,6 +41,99 @@ __global__ void eval_points_kernel(const uint64_t* __restrict__ tape, uint32_t n
     }
     out[i] = slots[i];
     (void)n_slots;
+}
+
+// Points with the slot file in shared memory, K per thread (rows of K floats,
+// [row][thread]: one access of up to 16 bytes per operand), over records that
+// the host makes of the tape (point_code: constants in the words that use them,
+// few rows), every branch the warp's. In global memory each word costs three accesses of the whole file
+// (270 MB for a million points and the 67 slots of a union of 64 spheres), and
+// the file has to be allocated: 1.61 -> 0.30 ms (with 13 slots and 2,900 words
+// 5.2 -> 0.90 ms), a thousand points 158 -> 48 us.
+constexpr uint32_t EVAL_THREADS = 64, EVAL_MAX_ROWS = 48;
+// A record: operand a, operand b (offset of the row, or a constant's bits), the
+// result's row, the operation with these bits.
+constexpr uint32_t EVAL_IMM_A = 1u << 8, EVAL_IMM_B = 1u << 9;
+
+template <int K>
+struct alignas(4 * K) Points {
+    float v[K];
+};
+
+// The operations that the loop below leaves out.
+template <int K>
+__device__ __noinline__ Points<K> eval_rare(uint32_t op, Points<K> a, Points<K> b) {
+#pragma unroll 1
+    for (int k = 0; k < K; k++) a.v[k] = pt_apply(op, 0, a.v[k], b.v[k]);
+    return a;
+}
+
+template <int K>
+__global__ void __launch_bounds__(EVAL_THREADS)
+    eval_points_shared_kernel(const uint4* __restrict__ recs, uint32_t n_recs, uint32_t result,
+                              const float4* __restrict__ xyzt, uint32_t n, float* __restrict__ out) {
+    extern __shared__ __align__(16) unsigned char eval_shared[];
+    uint4* const stage = reinterpret_cast<uint4*>(eval_shared) + (threadIdx.x & ~31u);
+    Points<K>* const s = reinterpret_cast<Points<K>*>(eval_shared + EVAL_THREADS * sizeof(uint4)) + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t first = (uint64_t)blockIdx.x * (EVAL_THREADS * K) + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const uint64_t i = first + (uint64_t)k * EVAL_THREADS;
+        const float4 p = xyzt[i < n ? i : n - 1];
+        s[0 * EVAL_THREADS].v[k] = p.x;
+        s[1 * EVAL_THREADS].v[k] = p.y;
+        s[2 * EVAL_THREADS].v[k] = p.z;
+        s[3 * EVAL_THREADS].v[k] = p.w;
+    }
+    uint4 next = lane < n_recs ? __ldg(&recs[lane]) : make_uint4(0, 0, 0, 0);
+    for (uint32_t base = 0; base < n_recs; base += 32) {
+        __syncwarp();
+        stage[lane] = next;
+        __syncwarp();
+        if (base + 32 + lane < n_recs) next = __ldg(&recs[base + 32 + lane]);
+        const uint32_t m = min(n_recs - base, 32u);
+        uint4 rec = stage[0];
+        for (uint32_t j = 0; j < m; j++) {
+            const uint4 q = rec;
+            rec = stage[(j + 1) & 31];
+            const uint32_t op = q.w & 0xFFu;
+            Points<K> a = s[q.w & EVAL_IMM_A ? 0u : q.x], b = s[q.w & EVAL_IMM_B ? 0u : q.y];
+#pragma unroll
+            for (int k = 0; k < K; k++) {
+                if (q.w & EVAL_IMM_A) a.v[k] = __uint_as_float(q.x);
+                if (q.w & EVAL_IMM_B) b.v[k] = __uint_as_float(q.y);
+            }
+            Points<K> r;
+            if (op == OP_MUL) {
+#pragma unroll
+                for (int k = 0; k < K; k++) r.v[k] = pt_apply(OP_MUL, 0, a.v[k], b.v[k]);
+            } else if (op == OP_ADD) {
+#pragma unroll
+                for (int k = 0; k < K; k++) r.v[k] = pt_apply(OP_ADD, 0, a.v[k], b.v[k]);
+            } else if (op == OP_SUB) {
+#pragma unroll
+                for (int k = 0; k < K; k++) r.v[k] = pt_apply(OP_SUB, 0, a.v[k], b.v[k]);
+            } else if (op == OP_MIN) {
+#pragma unroll
+                for (int k = 0; k < K; k++) r.v[k] = pt_apply(OP_MIN, 0, a.v[k], b.v[k]);
+            } else if (op == OP_MAX) {
+#pragma unroll
+                for (int k = 0; k < K; k++) r.v[k] = pt_apply(OP_MAX, 0, a.v[k], b.v[k]);
+            } else if (op == OP_NEG) {
+#pragma unroll
+                for (int k = 0; k < K; k++) r.v[k] = pt_apply(OP_NEG, 0, a.v[k], b.v[k]);
+            } else {
+                r = eval_rare<K>(op, a, b);
+            }
+            s[q.z] = r;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const uint64_t i = first + (uint64_t)k * EVAL_THREADS;
+        if (i < n) out[i] = s[result].v[k];
+    }
 }
 
 template <int ROUND>
@@ -117,11 +214,9 @@ struct EvalBuffers {
     }
 };
 
-frep_status eval_common(frep_ctx* ctx, const frep_tape* tape, uint32_t n, uint64_t in_bytes, uint64_t slot_bytes,
-                        uint64_t out_bytes, EvalBuffers* buf, uint8_t** in, uint8_t** slots, uint8_t** out,
-                        const char* who) {
-    // Every slot an instruction names must be a row of the slot file the
-    // kernels index with it.
+// Every slot an instruction names must be a row of the slot file the kernels
+// index with it.
+frep_status check_slots(const frep_tape* tape, const char* who) {
     const uint32_t n_slots = std::max<uint32_t>(tape->ct.n_slots, 4);
     for (const uint64_t w : tape->ct.instrs) {
         const uint32_t op = (uint32_t)w & 0xFFu, o = ((uint32_t)w >> 16) & 0xFFFFu;
@@ -130,7 +225,112 @@ frep_status eval_common(frep_ctx* ctx, const frep_tape* tape, uint32_t n, uint64
             (frep::dev::is_binary(op) && b >= n_slots))
             return fail(FREP_ERR_INVALID_ARG, "%s: instruction names a slot outside the tape's %u slots", who, n_slots);
     }
-    const uint64_t tape_bytes = align_up(tape->ct.instrs.size() * 8 + 8, 256);
+    return FREP_OK;
+}
+
+// The records of eval_points_shared_kernel for a checked tape: the same
+// operations on the same operands, without words for constants, in an order
+// that keeps few values at a time (operands right before their use, the one
+// that needs more rows first) and with rows given out by last use. A tape puts
+// the 64 spheres of a union first and their minima last: 67 slots, 9 rows.
+struct PointCode {
+    std::vector<uint4> recs;
+    uint32_t rows = 4, result = 0;  // rows of the slot file, offset of the result's
+};
+
+PointCode point_code(const std::vector<uint64_t>& instrs, uint32_t n_slots) {
+    constexpr uint32_t T = frep::dev::EVAL_THREADS, CONST = ~0u, INPUTS = 4;
+    struct Ref {
+        uint32_t value = CONST, bits = 0;  // a value's number, or a constant
+    };
+    struct Value {
+        uint32_t op = 0, need = 0, last = 0;
+        Ref a, b;
+        bool placed = false;
+    };
+    std::vector<Value> v(INPUTS);
+    std::vector<Ref> slot(n_slots);
+    for (uint32_t i = 0; i < INPUTS; i++) {
+        slot[i].value = i;
+        v[i].placed = true;
+    }
+    for (const uint64_t w : instrs) {
+        const uint32_t op = (uint32_t)w & 0xFFu, o = ((uint32_t)w >> 16) & 0xFFFFu;
+        if (op == FREP_TAPE_CONST) {
+            slot[o] = Ref{CONST, (uint32_t)(w >> 32)};
+            continue;
+        }
+        Value x;
+        x.op = op;
+        x.a = slot[(uint32_t)(w >> 32) & 0xFFFFu];
+        if (frep::dev::is_binary(op)) x.b = slot[(uint32_t)(w >> 48)];
+        const uint32_t na = x.a.value == CONST ? 0 : v[x.a.value].need, nb = x.b.value == CONST ? 0 : v[x.b.value].need;
+        x.need = std::max(1u, na == nb ? na + 1 : std::max(na, nb));
+        slot[o] = Ref{(uint32_t)v.size(), 0};
+        v.push_back(x);
+    }
+    if (slot[0].value < INPUTS || slot[0].value == CONST) {  // no operation left: copy it
+        Value x;
+        x.op = FREP_TAPE_COPY;
+        x.a = slot[0];
+        slot[0] = Ref{(uint32_t)v.size(), 0};
+        v.push_back(x);
+    }
+    // Depth first from the result.
+    const uint32_t result = slot[0].value;
+    std::vector<uint32_t> order, stack = {result};
+    while (!stack.empty()) {
+        const uint32_t i = stack.back();
+        if (v[i].placed) {
+            stack.pop_back();
+            continue;
+        }
+        const uint32_t a = v[i].a.value, b = v[i].b.value;
+        const bool wait_a = a != CONST && !v[a].placed, wait_b = b != CONST && !v[b].placed;
+        if (!wait_a && !wait_b) {
+            v[i].placed = true;
+            for (const uint32_t u : {a, b})
+                if (u != CONST) v[u].last = (uint32_t)order.size();
+            order.push_back(i);
+            stack.pop_back();
+        } else {  // the top of the stack is placed first
+            const bool a_first = wait_a && (!wait_b || v[a].need >= v[b].need);
+            if (a_first && wait_b) stack.push_back(b);
+            if (wait_a) stack.push_back(a);
+            if (!a_first && wait_b) stack.push_back(b);
+        }
+    }
+    PointCode code;
+    std::vector<uint32_t> row(v.size(), 0), free_rows;
+    for (uint32_t i = 0; i < INPUTS; i++) row[i] = i;
+    for (uint32_t at = 0; at < order.size(); at++) {
+        const Value& x = v[order[at]];
+        uint4 q = make_uint4(x.a.bits, x.b.bits, 0, x.op);
+        if (x.a.value == CONST) q.w |= frep::dev::EVAL_IMM_A;
+        else q.x = row[x.a.value] * T;
+        if (!frep::dev::is_binary(x.op)) q.y = 0;
+        else if (x.b.value == CONST) q.w |= frep::dev::EVAL_IMM_B;
+        else q.y = row[x.b.value] * T;
+        for (const uint32_t u : {x.a.value, x.b.value == x.a.value ? CONST : x.b.value})
+            if (u != CONST && u >= INPUTS && v[u].last == at) free_rows.push_back(row[u]);
+        if (free_rows.empty()) {
+            row[order[at]] = code.rows++;
+        } else {
+            row[order[at]] = free_rows.back();
+            free_rows.pop_back();
+        }
+        q.z = row[order[at]] * T;
+        code.recs.push_back(q);
+    }
+    code.result = row[result] * T;
+    return code;
+}
+
+// `code`: what the kernel runs (the tape's words, or records made of them).
+frep_status eval_common(frep_ctx* ctx, const void* code, uint64_t code_bytes, uint64_t in_bytes, uint64_t slot_bytes,
+                        uint64_t out_bytes, EvalBuffers* buf, uint8_t** in, uint8_t** slots, uint8_t** out,
+                        const char* who) {
+    const uint64_t tape_bytes = align_up(code_bytes + 8, 256);
     const uint64_t total = tape_bytes + align_up(in_bytes, 256) + align_up(slot_bytes, 256) + align_up(out_bytes, 256);
     if (ctx->used + total > ctx->budget)
         return fail(FREP_ERR_OOM, "%s: %llu bytes of working memory exceed the context's budget", who,
@@ -143,11 +343,10 @@ frep_status eval_common(frep_ctx* ctx, const frep_tape* tape, uint32_t n, uint64
                     cudaGetErrorString(e));
     }
     uint8_t* base = static_cast<uint8_t*>(buf->p);
-    FREP_CUDA(cudaMemcpy(base, tape->ct.instrs.data(), tape->ct.instrs.size() * 8, cudaMemcpyHostToDevice));
+    FREP_CUDA(cudaMemcpy(base, code, code_bytes, cudaMemcpyHostToDevice));
     *in = base + tape_bytes;
     *slots = *in + align_up(in_bytes, 256);
     *out = *slots + align_up(slot_bytes, 256);
-    (void)n;
     return FREP_OK;
 }
 
@@ -159,18 +358,40 @@ extern "C" frep_status frep_tape_eval_device(frep_ctx* ctx, const frep_tape* tap
     if (n == 0) return FREP_OK;
     if (tape->ct.instrs.empty()) return fail(FREP_ERR_INVALID_ARG, "frep_tape_eval_device: empty tape");
     const uint32_t n_slots = std::max<uint32_t>(tape->ct.n_slots, 4);
+    // Rows in shared memory while four blocks of four points per thread fit an
+    // SM (48 rows: 49 KB each); one point per thread until that many points
+    // give each SM two blocks of four (1,000 points: 48 against 66 us with four;
+    // 75,776: 68 and 67; 150,000: 110 against 76).
+    constexpr uint32_t T = frep::dev::EVAL_THREADS;
+    frep_status st = check_slots(tape, "frep_tape_eval_device");
+    if (st != FREP_OK) return st;
+    const PointCode pc = point_code(tape->ct.instrs, n_slots);
+    const bool shared = pc.rows <= frep::dev::EVAL_MAX_ROWS;
+    const uint32_t K = n >= 148u * 2 * T * 4 ? 4 : 1;
     EvalBuffers buf;
     uint8_t *d_in, *d_slots, *d_out;
-    frep_status st = eval_common(ctx, tape, n, (uint64_t)n * 16, (uint64_t)n * n_slots * 4, (uint64_t)n * 4, &buf,
-                                 &d_in, &d_slots, &d_out, "frep_tape_eval_device");
+    const void* code = shared ? static_cast<const void*>(pc.recs.data()) : tape->ct.instrs.data();
+    const uint64_t code_bytes = shared ? pc.recs.size() * sizeof(uint4) : tape->ct.instrs.size() * 8;
+    st = eval_common(ctx, code, code_bytes, (uint64_t)n * 16, shared ? 0 : (uint64_t)n * n_slots * 4, (uint64_t)n * 4,
+                     &buf, &d_in, &d_slots, &d_out, "frep_tape_eval_device");
     if (st != FREP_OK) return st;
     FREP_CUDA(cudaMemcpy(d_in, xyzt, (size_t)n * 16, cudaMemcpyHostToDevice));
-    const uint32_t threads = 128, blocks = (n + threads - 1) / threads;
-    frep::dev::eval_points_kernel<<<blocks, threads>>>(static_cast<const uint64_t*>(buf.p),
-                                                        (uint32_t)tape->ct.instrs.size(), n_slots,
-                                                        reinterpret_cast<const float4*>(d_in), n,
-                                                        reinterpret_cast<float*>(d_slots),
-                                                        reinterpret_cast<float*>(d_out));
+    const auto* d_xyzt = reinterpret_cast<const float4*>(d_in);
+    if (shared) {
+        const uint32_t blocks = (uint32_t)(((uint64_t)n + T * K - 1) / (T * K));
+        const uint32_t bytes = T * 16 + pc.rows * T * K * 4;
+        const auto kernel = K == 4 ? frep::dev::eval_points_shared_kernel<4> : frep::dev::eval_points_shared_kernel<1>;
+        FREP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(T * 16 + frep::dev::EVAL_MAX_ROWS * T * K * 4)));
+        kernel<<<blocks, T, bytes>>>(static_cast<const uint4*>(buf.p), (uint32_t)pc.recs.size(), pc.result, d_xyzt,
+                                     n, reinterpret_cast<float*>(d_out));
+    } else {
+        const uint32_t threads = 128, blocks = (n + threads - 1) / threads;
+        frep::dev::eval_points_kernel<<<blocks, threads>>>(static_cast<const uint64_t*>(buf.p),
+                                                            (uint32_t)tape->ct.instrs.size(), n_slots, d_xyzt, n,
+                                                            reinterpret_cast<float*>(d_slots),
+                                                            reinterpret_cast<float*>(d_out));
+    }
     FREP_CUDA(cudaGetLastError());
     FREP_CUDA(cudaMemcpy(out, d_out, (size_t)n * 4, cudaMemcpyDeviceToHost));
     return FREP_OK;
@@ -187,8 +408,11 @@ extern "C" frep_status frep_tape_eval_intervals(frep_ctx* ctx, const frep_tape* 
     EvalBuffers buf;
     uint8_t *d_in, *d_slots, *d_out;
     const uint64_t row_bytes = rounding == FREP_ROUND_HYBRID ? 32 : 8;
-    frep_status st = eval_common(ctx, tape, n, (uint64_t)n * 24, (uint64_t)n * n_slots * row_bytes, (uint64_t)n * 8,
-                                 &buf, &d_in, &d_slots, &d_out, "frep_tape_eval_intervals");
+    frep_status st = check_slots(tape, "frep_tape_eval_intervals");
+    if (st != FREP_OK) return st;
+    st = eval_common(ctx, tape->ct.instrs.data(), tape->ct.instrs.size() * 8, (uint64_t)n * 24,
+                     (uint64_t)n * n_slots * row_bytes, (uint64_t)n * 8, &buf, &d_in, &d_slots, &d_out,
+                     "frep_tape_eval_intervals");
     if (st != FREP_OK) return st;
     FREP_CUDA(cudaMemcpy(d_in, boxes, (size_t)n * 24, cudaMemcpyHostToDevice));
     const uint32_t threads = 128, blocks = (n + threads - 1) / threads;
