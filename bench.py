@@ -430,7 +430,7 @@ def run_ours(args, world, rank, local):
     fp32_peak_tops = SM_COUNT * FP32_LANES_PER_SM * sm_mhz * 1e6 / 1e12
     achieved = fp32_ops[dom] / (level_ms[dom] / 1e3) / 1e12
     roofline = {
-        "bound": "fp32", "kernel": "point_level_kernel" if dom == vs.grid_levels - 1 else "interval_level_kernel",
+        "bound": "fp32", "kernel": "last-level pass" if dom == vs.grid_levels - 1 else "interval_level_kernel",
         "level": dom, "achieved": achieved, "peak": fp32_peak_tops, "unit": "TFLOP/s",
         "frac": achieved / fp32_peak_tops, "traffic": None,
         "peak_source": "nominal FP32 issue: 148 SMs x 128 lanes x MEASURED_PEAKS.json sm_max_mhz "
@@ -894,7 +894,7 @@ def run_ours_batch(args, world, rank, local):
     sm_mhz = float(peaks.get("sm_max_mhz", 1965.0))
     fp32_peak = SM_COUNT * FP32_LANES_PER_SM * sm_mhz * 1e6 / 1e12
     achieved = float(ops[dom]) / (dom_ms / 1e3) / 1e12
-    kind_name = ["interval_level_kernel", "point_level_kernel (4 cells/lane)", "point_level_kernel (2 cells/lane)"]
+    kind_name = ["interval_level_kernel", "last-level pass (trees with 4 cells/lane)", "last-level pass (2 cells/lane)"]
     total_ops = float(ops.sum())
     default_workload = (n == 512 and (W, H) == (512, 512) and not args.tune_cache and not args.retune
                         and tuning_table() is not None)
