@@ -415,7 +415,7 @@ frep_status ensure_plan(frep_tree* tree, const frep_tape* tape, const char* who)
 frep_status enqueue_tree_levels(frep_tree* tree, const frep_tape* tape, float tape_time, uint32_t* keep,
                                 frep::WarpScratch ws, const frep::LevelPlan& plan, cudaStream_t stream,
                                 const frep_tree* prev = nullptr) {
-    cudaError_t e = frep::launch_tree_init(tree->d_self, 1, nullptr, tape_time, stream);
+    cudaError_t e = frep::launch_tree_init(tree->d_self, 1, nullptr, tape_time, tape->transcendental, stream);
     if (e != cudaSuccess) return cuda_fail(e, "tree_init_kernel");
     if (prev) {
         e = frep::launch_reuse_match(tree->hdr, prev->hdr, tree->reuse_src, tree->reuse_list, 0, stream);

@@ -65,8 +65,7 @@ struct frep_tape {
     void build_record() {
         transcendental = false;
         for (const uint64_t w : ct.instrs) {
-            const uint32_t op = frep::dev::w_op_host(w);
-            transcendental |= op == frep::dev::OP_SIN || op == frep::dev::OP_COS || op == frep::dev::OP_EXP;
+            transcendental |= frep::dev::is_transcendental(frep::dev::w_op_host(w));
         }
         record.assign(frep::detail::align_up(1 + ct.instrs.size(), frep::dev::TAPE_ALIGN_WORDS), 0);
         record[0] = ct.instrs.size();

@@ -38,6 +38,7 @@ struct TreeHeader {
     uint32_t point_k;                          // last-level pass: cells per lane (2 or 4)
     // ---- per voxelization ----
     float tape_time;
+    uint32_t transcendental;                   // the root tape has SIN, COS or EXP
     uint32_t node_count[MAX_LEVELS];           // interiorNodeCount
     unsigned long long node_ofs[MAX_LEVELS];   // u32 words
     unsigned long long tape_top;               // u64 words
@@ -80,6 +81,9 @@ __host__ __device__ inline uint32_t node_words(uint32_t dim, bool last) {
 __device__ __constant__ const uint8_t kIntervalOps[16] = {0, 18, 18, 2, 2, 10, 16, 4, 4, 2, 0, 4, 0, 0, 0, 0};
 __device__ __constant__ const uint8_t kPointOps[16]    = {0, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 0, 0, 0, 0};
 
+__host__ __device__ constexpr bool is_transcendental(uint32_t op) {
+    return op == OP_SIN || op == OP_COS || op == OP_EXP;
+}
 inline uint32_t w_op_host(uint64_t w) { return (uint32_t)w & 0xFFu; }
 __device__ __forceinline__ uint32_t w_op(uint64_t w) { return (uint32_t)w & 0xFFu; }
 __device__ __forceinline__ uint32_t w_out(uint64_t w) { return ((uint32_t)w >> 16) & 0xFFFFu; }

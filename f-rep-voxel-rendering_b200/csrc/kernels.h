@@ -130,9 +130,10 @@ inline uint64_t fine_cells(const uint32_t* dims, uint32_t levels) {
 
 // Resets the headers of n trees (tape time from `tape_times`, or `tape_time`
 // when it is null) and writes their root nodes. Each tree's root tape must
-// already be at word 0 of its tape pool.
+// already be at word 0 of its tape pool. transcendental: whether any of them has
+// a SIN, COS or EXP.
 cudaError_t launch_tree_init(dev::TreeHeader* const* trees, uint32_t n, const float* tape_times, float tape_time,
-                             cudaStream_t stream);
+                             bool transcendental, cudaStream_t stream);
 // Same for a batch whose root tapes are staged in one device buffer: tree i's
 // record is words [offsets[i], offsets[i+1]) of `staged`; it is copied to
 // word 0 of the tree's pool first. tape_times has n entries.

@@ -835,6 +835,7 @@ __device__ __forceinline__ bool iv_micro_forward(const uint64_t* tape, uint32_t 
 // 17-31 its length (item tapes of 2^15 words or more are not stored; the
 // scratch holds at most kItemTapeWords <= 2^19 words).
 struct ItemNode {  // the node of a group of items, and its tree's frame
+    const TreeHeader* H;
     uint32_t dim, dim_sh, ncx, ncy, ncz;
     float cs, lx, ly, lz, tt;
 };
@@ -848,13 +849,13 @@ __device__ __noinline__ uint32_t prepare_items(const uint64_t* tape, uint32_t n,
     const uint32_t dim = T.dim, ncx = T.ncx, ncy = T.ncy, ncz = T.ncz;
     const bool valid = lane < g;
     // a tape with SIN / COS / EXP: the whole group runs the node's tape (found
-    // before anything is evaluated)
-    bool trans = false;
-    for (uint32_t i = lane; i < n; i += 32) {
-        const uint32_t op = w_op(__ldcg(&tape[i]));
-        trans |= op == OP_SIN || op == OP_COS || op == OP_EXP;
+    // before anything is evaluated, and looked for only where the tree's root
+    // tape has one: shortening adds none)
+    if (T.H->transcendental) {
+        bool trans = false;
+        for (uint32_t i = lane; i < n; i += 32) trans |= is_transcendental(w_op(__ldcg(&tape[i])));
+        if (__any_sync(0xFFFFFFFFu, trans)) return 0u;
     }
-    if (__any_sync(0xFFFFFFFFu, trans)) return 0u;
     // the item is a brick (brick_origin): its cells' bounding box
     uint32_t x0, y0, z0;
     brick_origin<KI>(grp + (valid ? lane : 0u), dim, T.dim_sh, &x0, &y0, &z0);
@@ -1079,7 +1080,7 @@ interval_level_kernel(LevelLaunch p) {
                         // the rest of this node's items in the fetched chunk, up to 32
                         const uint32_t g = min(min(32u, groups - grp), got - it);
                         p_plan = prepare_items<ROUND, KI>(
-                            tape, n_node, ItemNode{dim, T.dim_sh, ncx, ncy, ncz, cs, T.lx, T.ly, T.lz, T.tt}, grp, g,
+                            tape, n_node, ItemNode{T.H, dim, T.dim_sh, ncx, ncy, ncz, cs, T.lx, T.ly, T.lz, T.tt}, grp, g,
                             smem_addr(wbase) + lane * 8u, stage, keep, mmb, items, p.mm_cap, p.n_slots,
                             p.item_cap);
                         pg_first = item;
@@ -1907,7 +1908,8 @@ __device__ __forceinline__ void zero_root_masks(TreeHeader* H, uint32_t t, uint3
 // Resets the headers and writes the root nodes (Voxelizer::Voxelize sets
 // interiorNodeCount[0] = 1 and relies on a zeroed root, voxelizer.cpp:432-435).
 // One block per tree; each tree's root tape is already at word 0 of its pool.
-__global__ void tree_init_kernel(TreeHeader* const* trees, uint32_t n, const float* tape_times, float tape_time) {
+__global__ void tree_init_kernel(TreeHeader* const* trees, uint32_t n, const float* tape_times, float tape_time,
+                                 uint32_t transcendental) {
     for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
         TreeHeader* H = trees[i];
         const uint32_t t = threadIdx.x;
@@ -1926,6 +1928,7 @@ __global__ void tree_init_kernel(TreeHeader* const* trees, uint32_t n, const flo
             H->overflow = 0;
             H->status = 0;
             H->tape_time = tape_times ? tape_times[i] : tape_time;
+            H->transcendental = transcendental;
             uint32_t* root = H->nodes;
             root[0] = 0;  // root tape at word 0 of the tape pool
             root[1] = 0;
@@ -1945,8 +1948,13 @@ __global__ void tree_init_staged_kernel(TreeHeader* const* trees, uint32_t n, co
         TreeHeader* H = trees[i];
         uint64_t* pool = H->tapes;
         const unsigned long long b = offsets[i], e = offsets[i + 1];
-        for (unsigned long long w = b + threadIdx.x; w < e; w += blockDim.x) pool[w - b] = staged[w];
-        __syncthreads();
+        bool trans = false;
+        for (unsigned long long w = b + threadIdx.x; w < e; w += blockDim.x) {
+            const uint64_t v = staged[w];
+            pool[w - b] = v;
+            trans |= w > b && is_transcendental(w_op(v));  // (word 0: the count; padding: zeros)
+        }
+        const uint32_t transcendental = __syncthreads_or(trans) ? 1u : 0u;
         const uint32_t t = threadIdx.x;
         const uint32_t root_n = (uint32_t)pool[0];
         if (t < MAX_LEVELS) {
@@ -1963,6 +1971,7 @@ __global__ void tree_init_staged_kernel(TreeHeader* const* trees, uint32_t n, co
             H->overflow = 0;
             H->status = 0;
             H->tape_time = tape_times[i];
+            H->transcendental = transcendental;
             uint32_t* root = H->nodes;
             root[0] = 0;
             root[1] = 0;
@@ -2138,9 +2147,9 @@ cudaError_t plan_levels(uint32_t n_slots, uint32_t mm_cap, int point_k, int roun
 }
 
 cudaError_t launch_tree_init(dev::TreeHeader* const* trees, uint32_t n, const float* tape_times, float tape_time,
-                             cudaStream_t stream) {
+                             bool transcendental, cudaStream_t stream) {
     const uint32_t blocks = n < 4096 ? n : 4096;
-    dev::tree_init_kernel<<<blocks, 32, 0, stream>>>(trees, n, tape_times, tape_time);
+    dev::tree_init_kernel<<<blocks, 32, 0, stream>>>(trees, n, tape_times, tape_time, transcendental ? 1u : 0u);
     return cudaGetLastError();
 }
 
