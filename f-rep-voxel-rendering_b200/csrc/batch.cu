@@ -142,7 +142,8 @@ frep_status acquire_area(frep_batch* b, size_t bytes, int* which, cudaStream_t s
         if (old_d) FREP_CUDA(cudaFreeAsync(old_d, s));
         // (each growth costs allocations and a new graph capture: at least twofold)
         const size_t cap = align_up(std::max(bytes + bytes / 4, 2 * prev), 4096);
-        if (b->ctx->used + cap > b->ctx->budget) return fail(FREP_ERR_OOM, "frep_batch: upload area exceeds the budget");
+        if (!frep::detail::reserve(b->ctx, cap))
+            return fail(FREP_ERR_OOM, "frep_batch: upload area exceeds the budget");
         FREP_CUDA(cudaMallocHost(&A.h, cap));
         FREP_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&A.d), cap, s));
         A.bytes = cap;
@@ -193,8 +194,9 @@ frep_status ensure_keep(frep_batch* b, uint64_t words) {
         b->keep = nullptr;
         b->keep_words = 0;
     }
-    if (b->ctx->used + words * 4 > b->ctx->budget) return fail(FREP_ERR_OOM, "frep_batch: scratch exceeds the budget");
-    FREP_CUDA(cudaMalloc(&b->keep, words * 4));
+    if (!frep::detail::reserve(b->ctx, words * 4))
+        return fail(FREP_ERR_OOM, "frep_batch: scratch exceeds the budget");
+    FREP_CUDA(frep::detail::device_alloc(b->ctx, (void**)&b->keep, words * 4));
     b->keep_words = words;
     b->bytes += words * 4;
     b->ctx->used += words * 4;

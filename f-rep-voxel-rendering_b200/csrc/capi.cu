@@ -158,7 +158,11 @@ frep_status frep_ctx_create(int device, uint64_t hbm_budget_bytes, frep_ctx** ou
     return FREP_OK;
 }
 
-void frep_ctx_destroy(frep_ctx* ctx) { delete ctx; }
+void frep_ctx_destroy(frep_ctx* ctx) {
+    if (!ctx) return;
+    for (frep_tree* t : ctx->spare) t->spare = false;
+    delete ctx;
+}
 
 frep_status frep_ctx_memory(const frep_ctx* ctx, uint64_t* used, uint64_t* budget) {
     if (!ctx) return fail(FREP_ERR_INVALID_ARG, "frep_ctx_memory: null argument");
@@ -198,6 +202,64 @@ __global__ void tree_header_write_kernel(const TreeHeader h, TreeHeader* dst, Tr
 }  // namespace dev
 
 namespace detail {
+
+namespace {
+
+// Puts the tree into its context's list or takes it out.
+void set_spare(frep_tree* t, bool spare) {
+    if (t->spare == spare) return;
+    std::lock_guard<std::recursive_mutex> lock(t->ctx->spare_mu);
+    auto& list = t->ctx->spare;
+    if (spare) list.push_back(t);
+    else list.erase(std::remove(list.begin(), list.end(), t), list.end());
+    t->spare = spare;
+}
+
+// Gives back what the listed trees' scratch holds beyond their need.
+void release_spare(frep_ctx* ctx) {
+    if (ctx->spare.empty() || cudaSetDevice(ctx->device) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) return;
+    for (frep_tree* t : ctx->spare) {
+        const uint64_t need = t->keep_need;
+        cudaFree(t->keep);
+        t->keep = nullptr;
+        if (cudaMalloc(&t->keep, need * 4) != cudaSuccess) {
+            cudaGetLastError();
+            t->keep = nullptr;  // (its next voxelization allocates)
+        }
+        const uint64_t freed = (t->keep_words - (t->keep ? need : 0)) * 4;
+        t->keep_words = t->keep ? need : 0;
+        t->spare = false;
+        t->bytes -= freed;
+        ctx->used -= std::min(ctx->used, freed);
+    }
+    ctx->spare.clear();
+}
+
+}  // namespace
+
+uint64_t budget_left(frep_ctx* ctx) {
+    std::lock_guard<std::recursive_mutex> lock(ctx->spare_mu);
+    uint64_t used = ctx->used;
+    for (const frep_tree* t : ctx->spare) used -= std::min(used, (t->keep_words - t->keep_need) * 4);
+    return ctx->budget > used ? ctx->budget - used : 0;
+}
+
+bool reserve(frep_ctx* ctx, uint64_t bytes) {
+    std::lock_guard<std::recursive_mutex> lock(ctx->spare_mu);
+    if (ctx->used + bytes <= ctx->budget) return true;
+    if (bytes <= budget_left(ctx)) release_spare(ctx);
+    return ctx->used + bytes <= ctx->budget;
+}
+
+cudaError_t device_alloc(frep_ctx* ctx, void** p, uint64_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    std::lock_guard<std::recursive_mutex> lock(ctx->spare_mu);
+    if (ctx->spare.empty()) return e;
+    cudaGetLastError();
+    release_spare(ctx);
+    return cudaMalloc(p, bytes);
+}
 
 uint64_t tree_external_bytes(uint64_t node_words, uint64_t tape_words) {
     return align_up(sizeof(dev::TreeHeader), 256) + 256 + align_up(node_words * 4, 256) + tape_words * 8;
@@ -255,7 +317,7 @@ frep_status tree_create_impl(frep_ctx* ctx, const frep_grid* grid, const frep_vo
         dense_nodes = std::min<uint64_t>(dense_nodes * d3, 1ull << 40);
         dense_words = std::min<uint64_t>(dense_words, 1ull << 44);
     }
-    const uint64_t avail = ext ? ext_bytes : (ctx->budget > ctx->used ? ctx->budget - ctx->used : 0);
+    const uint64_t avail = ext ? ext_bytes : budget_left(ctx);
     if (ext && (!t->opts.node_words || !t->opts.tape_words)) {
         delete t;
         return fail(FREP_ERR_INVALID_ARG, "tree in caller memory: pool sizes must be given");
@@ -265,7 +327,7 @@ frep_status tree_create_impl(frep_ctx* ctx, const frep_grid* grid, const frep_vo
     t->tape_cap = std::min<uint64_t>(t->tape_cap, 0xFFFFFFF0ull);  // tape indices are u32
     const uint64_t bytes = ext ? tree_external_bytes(t->node_cap, t->tape_cap)
                                : t->node_cap * 4 + t->tape_cap * 8 + sizeof(frep::dev::TreeHeader);
-    if (t->node_cap < t->node_size[0] || bytes > avail) {
+    if (t->node_cap < t->node_size[0] || bytes > avail || (!ext && !reserve(ctx, bytes))) {
         delete t;
         return fail(FREP_ERR_OOM, "frep_tree_create: %llu bytes requested, %llu left in the budget",
                     (unsigned long long)bytes, (unsigned long long)avail);
@@ -277,10 +339,10 @@ frep_status tree_create_impl(frep_ctx* ctx, const frep_grid* grid, const frep_vo
         t->nodes = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(t->d_small) + 256);
         t->tapes = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(t->nodes) + align_up(t->node_cap * 4, 256));
     } else {
-        e = cudaMalloc(&t->hdr, sizeof(frep::dev::TreeHeader));
-        if (e == cudaSuccess) e = cudaMalloc(&t->d_small, 64);
-        if (e == cudaSuccess) e = cudaMalloc(&t->nodes, t->node_cap * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&t->tapes, t->tape_cap * 8);
+        e = device_alloc(ctx, (void**)&t->hdr, sizeof(frep::dev::TreeHeader));
+        if (e == cudaSuccess) e = device_alloc(ctx, (void**)&t->d_small, 64);
+        if (e == cudaSuccess) e = device_alloc(ctx, (void**)&t->nodes, t->node_cap * 4);
+        if (e == cudaSuccess) e = device_alloc(ctx, (void**)&t->tapes, t->tape_cap * 8);
     }
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&t->upload_done, cudaEventDisableTiming);
     if (e != cudaSuccess) {
@@ -372,6 +434,7 @@ void frep_tree_destroy(frep_tree* t) {
         cudaFree(t->nodes);
         cudaFree(t->tapes);
     }
+    frep::detail::set_spare(t, false);
     cudaFree(t->keep);
     cudaFree(t->reuse_src);
     if (t->staging) cudaFreeHost(t->staging);
@@ -506,6 +569,18 @@ frep_status voxelize_impl(frep_ctx* ctx, frep_tree* tree, const frep_tree* prev,
 
     frep_status pst = ensure_plan(tree, tape, "frep_voxelize");
     if (pst != FREP_OK) return pst;
+    std::lock_guard<std::recursive_mutex> lock(ctx->spare_mu);
+    if (prev && !tree->reuse_src) {  // one entry per possible node (nodes are >= 8 words), twice
+        const uint64_t words = tree->node_cap / 8 + 1;
+        if (!frep::detail::reserve(ctx, words * 8))
+            return fail(FREP_ERR_OOM, "frep_voxelize_reuse: side arrays of %llu bytes exceed the budget",
+                        (unsigned long long)words * 8);
+        FREP_CUDA(frep::detail::device_alloc(ctx, (void**)&tree->reuse_src, words * 8));
+        tree->reuse_list = tree->reuse_src + words;
+        tree->reuse_words = words;
+        tree->bytes += words * 8;
+        ctx->used += words * 8;
+    }
     // Per-warp scratch: a keep mask per instruction, a choice-mask pair per
     // MIN/MAX, and room for item tapes (item-level pruning): as much as is at
     // most a quarter of the tree's own pools and the context's budget holds,
@@ -513,60 +588,65 @@ frep_status voxelize_impl(frep_ctx* ctx, frep_tree* tree, const frep_tree* prev,
     // node's tape); below that, and for tapes with transcendentals, which are
     // not pruned, the passes run without item pruning (the same trees). Each
     // tree keeps its scratch between voxelizations, so the bound keeps many
-    // small resident trees from each holding item room.
+    // small resident trees from each holding item room, and what it holds beyond
+    // the masks gives way to other allocations (release_spare).
     // (The 2048^3 scene's fitted pools give 1,500 words per warp: its level-1
     // pass took 1.76 ms without item pruning, 1.27 with; a 75-primitive scene's
     // at 12 x 20 x 4 with 1,100 words 2.26 and 1.02 ms.)
     const uint64_t warps = (uint64_t)tree->plan.blocks * tree->plan.warps_per_block;
     const uint32_t ki = (uint32_t)tree->plan.interval_ki;
-    frep::WarpScratch ws = frep::warp_scratch(n, tape->ct.n_minmax, ki);
+    const frep::WarpScratch plain = frep::warp_scratch(n, tape->ct.n_minmax, ki);
+    frep::WarpScratch ws = plain;
+    const uint64_t others = ctx->used - std::min<uint64_t>(ctx->used, tree->keep_words * 4);  // charged without the scratch
     if (tree->opts.rounding != FREP_ROUND_HYBRID && !tape->transcendental && tree->prune_items) {
         const uint64_t room = (tree->node_cap * 4 + tree->tape_cap * 8) / 4 / 8 / warps;  // words per warp
         uint32_t cap = (uint32_t)std::min<uint64_t>(room / 16 * 16, frep::kTreeItemTapeWords);
         for (; cap >= frep::kMinItemTapeWords; cap = cap / 2 / 16 * 16) {
             const frep::WarpScratch w = frep::warp_scratch(n, tape->ct.n_minmax, ki, cap);
-            const bool fits = warps * w.stride <= tree->keep_words ||
-                              ctx->used - std::min<uint64_t>(ctx->used, tree->keep_words * 4) + warps * w.stride * 4 <=
-                                  ctx->budget;
-            if (!fits) continue;
+            if (warps * w.stride > tree->keep_words && others + warps * w.stride * 4 > ctx->budget) continue;
             ws = w;
             break;
         }
     }
+    const uint64_t need = warps * plain.stride;
     uint64_t keep_words = warps * ws.stride;
     if (keep_words > tree->keep_words) {
         // (a tree that sees ever longer tapes, as when pools are fitted, grows it
         // by half at least, within the budget: each growth waits for the stream)
         const uint64_t grown = tree->keep_words + tree->keep_words / 2;
-        if (grown > keep_words &&
-            ctx->used - std::min<uint64_t>(ctx->used, tree->keep_words * 4) + grown * 4 <= ctx->budget)
-            keep_words = grown;
+        if (grown > keep_words && others + grown * 4 <= ctx->budget) keep_words = grown;
         if (tree->keep) {
             cudaStreamSynchronize(tree->stream);
             cudaFree(tree->keep);
-            tree->ctx->used -= std::min<uint64_t>(tree->ctx->used, tree->keep_words * 4);
+            ctx->used = others;
             tree->bytes -= tree->keep_words * 4;
+            frep::detail::set_spare(tree, false);
         }
         tree->keep = nullptr;
         tree->keep_words = 0;
-        if (ctx->used + keep_words * 4 > ctx->budget)
+        if (!frep::detail::reserve(ctx, keep_words * 4))
             return fail(FREP_ERR_OOM, "frep_voxelize: scratch of %llu bytes exceeds the budget", (unsigned long long)keep_words * 4);
-        FREP_CUDA(cudaMalloc(&tree->keep, keep_words * 4));
+        cudaError_t e = frep::detail::device_alloc(ctx, (void**)&tree->keep, keep_words * 4);
+        if (e == cudaErrorMemoryAllocation && keep_words > need) {  // the device holds less than the budget: no room
+            cudaGetLastError();
+            ws = plain;
+            keep_words = need;
+            e = cudaMalloc(&tree->keep, keep_words * 4);
+        }
+        if (e != cudaSuccess) tree->keep = nullptr;
+        FREP_CUDA(e);
         tree->keep_words = keep_words;
         tree->bytes += keep_words * 4;
         ctx->used += keep_words * 4;
+        tree->keep_captured = false;
     }
-    if (prev && !tree->reuse_src) {  // one entry per possible node (nodes are >= 8 words), twice
-        const uint64_t words = tree->node_cap / 8 + 1;
-        if (ctx->used + words * 8 > ctx->budget)
-            return fail(FREP_ERR_OOM, "frep_voxelize_reuse: side arrays of %llu bytes exceed the budget",
-                        (unsigned long long)words * 8);
-        FREP_CUDA(cudaMalloc(&tree->reuse_src, words * 8));
-        tree->reuse_list = tree->reuse_src + words;
-        tree->reuse_words = words;
-        tree->bytes += words * 8;
-        ctx->used += words * 8;
+    tree->keep_need = std::max(tree->keep_need, need);
+    if (tree->keep_words > tree->keep_need && !tree->keep_captured) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        FREP_CUDA(cudaStreamIsCapturing(stream, &capture));
+        tree->keep_captured = capture != cudaStreamCaptureStatusNone;
     }
+    frep::detail::set_spare(tree, tree->keep_words > tree->keep_need && !tree->keep_captured);
     // Root tape upload through pinned staging (reused once the previous copy is done).
     if (root_words > tree->staging_words) {
         if (tree->staging) {

@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -45,6 +46,14 @@ frep_status fill_render_args(const frep_tree* tree, const frep_camera* cam, cons
 // The frame part alone (camera basis, lights, outputs): resets *args first.
 frep_status fill_view_args(const frep_camera* cam, const frep_lights* lights, float tape_time,
                            const frep_image* out, RenderArgs* args);
+// Device memory of a context. Trees may hold more scratch than their passes need
+// (item room, growth by half): it gives way before an allocation is refused.
+// What of the budget is free, or would be without it:
+uint64_t budget_left(frep_ctx* ctx);
+// Whether `bytes` more fit the budget, after giving that scratch back if need be.
+bool reserve(frep_ctx* ctx, uint64_t bytes);
+// cudaMalloc, tried again after giving it back; counts nothing.
+cudaError_t device_alloc(frep_ctx* ctx, void** p, uint64_t bytes);
 // Host time of a batch's last frep_batch_voxelize, ms: plans, prefix and
 // scratch; the upload area; staging and launches.
 void batch_host_ms(const frep_batch* b, double out[3]);
@@ -78,6 +87,10 @@ struct frep_ctx {
     uint64_t budget = 0;
     uint64_t used = 0;
     int sm_count = 0;
+    // Trees whose scratch can give way (frep_tree::spare). The mutex is for a
+    // server on this context, whose scheduler allocates on a thread of its own.
+    std::vector<frep_tree*> spare;
+    std::recursive_mutex spare_mu;
 };
 
 struct frep_tree {
@@ -104,6 +117,9 @@ struct frep_tree {
     uint64_t node_cap = 0, tape_cap = 0;
     uint32_t* keep = nullptr;
     uint64_t keep_words = 0;
+    uint64_t keep_need = 0;      // of them, what its passes could not do without
+    bool keep_captured = false;  // a captured launch holds `keep`: it stays
+    bool spare = false;          // keep_words > keep_need and not captured: in the context's list
     uint64_t bytes = 0;
     // staging for the root tape upload
     uint64_t* staging = nullptr;

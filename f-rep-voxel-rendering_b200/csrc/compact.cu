@@ -32,7 +32,9 @@
 
 using frep::detail::align_up;
 using frep::detail::cuda_fail;
+using frep::detail::device_alloc;
 using frep::detail::fail;
+using frep::detail::reserve;
 
 struct frep_compact {
     frep_ctx* ctx = nullptr;
@@ -371,7 +373,9 @@ void compact_geometry(frep_compact* c) {
 
 // RAII for the temporary device buffers of one compaction.
 struct DevBufs {
+    frep_ctx* ctx;
     std::vector<void*> ptrs;
+    explicit DevBufs(frep_ctx* c) : ctx(c) {}
     ~DevBufs() {
         for (void* p : ptrs) cudaFree(p);
     }
@@ -383,7 +387,7 @@ struct DevBufs {
     template <typename T>
     cudaError_t alloc(T** p, uint64_t count) {
         *p = nullptr;
-        cudaError_t e = cudaMalloc((void**)p, std::max<uint64_t>(count, 1) * sizeof(T));
+        cudaError_t e = device_alloc(ctx, (void**)p, std::max<uint64_t>(count, 1) * sizeof(T));
         if (e == cudaSuccess) ptrs.push_back(*p);
         return e;
     }
@@ -456,12 +460,12 @@ frep_status frep_tree_compact(frep_ctx* ctx, frep_tree* tree, uint32_t mode, voi
     // tape slots) plus room for an exactly sized copy of the result.
     const uint64_t scratch =
         2 * (node_bound * 4 + tape_top * 8) + max_count * 16 + sum_count + (uint64_t)slots * 8;
-    if (ctx->used + scratch > ctx->budget)
+    if (!reserve(ctx, scratch))
         return fail(FREP_ERR_OOM, "frep_tree_compact: %llu bytes of working memory exceed the budget",
                     (unsigned long long)scratch);
 
     FREP_CUDA(cudaSetDevice(ctx->device));
-    DevBufs tmp;
+    DevBufs tmp(ctx);
     uint32_t *dnodes, *order0, *order1, *cnt, *base, *mark, *newofs, *partials;
     uint64_t* dtapes;
     uint8_t* status;
@@ -563,10 +567,10 @@ frep_status frep_tree_compact(frep_ctx* ctx, frep_tree* tree, uint32_t mode, voi
     // kept, a larger one is copied into an exact one (and released on return).
     e = cudaSuccess;
     if (c->node_words == node_bound) c->nodes = (uint32_t*)tmp.take(dnodes);
-    else e = cudaMalloc(&c->nodes, std::max<uint64_t>(c->node_words, 1) * 4);
+    else e = device_alloc(ctx, (void**)&c->nodes, std::max<uint64_t>(c->node_words, 1) * 4);
     if (e == cudaSuccess) {
         if (c->tape_words == tape_top) c->tapes = (uint64_t*)tmp.take(dtapes);
-        else e = cudaMalloc(&c->tapes, std::max<uint64_t>(c->tape_words, 1) * 8);
+        else e = device_alloc(ctx, (void**)&c->tapes, std::max<uint64_t>(c->tape_words, 1) * 8);
     }
     if (e == cudaSuccess && c->nodes != dnodes)
         e = cudaMemcpyAsync(c->nodes, dnodes, c->node_words * 4, cudaMemcpyDeviceToDevice, stream);
@@ -755,7 +759,7 @@ frep_status frep_compact_import(frep_ctx* ctx, const void* blob, uint64_t size, 
     frep_compact_header h;
     std::memcpy(&h, blob, sizeof(h));
     const uint64_t bytes = h.node_words * 4 + h.tape_words * 8;
-    if (ctx->used + bytes > ctx->budget)
+    if (!reserve(ctx, bytes))
         return fail(FREP_ERR_OOM, "frep_compact_import: %llu bytes exceed the budget", (unsigned long long)bytes);
     FREP_CUDA(cudaSetDevice(ctx->device));
     auto* c = new frep_compact();
@@ -776,8 +780,8 @@ frep_status frep_compact_import(frep_ctx* ctx, const void* blob, uint64_t size, 
     c->node_words = h.node_words;
     c->tape_words = h.tape_words;
     const uint8_t* p = (const uint8_t*)blob;
-    cudaError_t e = cudaMalloc(&c->nodes, std::max<uint64_t>(h.node_words, 1) * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&c->tapes, h.tape_words * 8);
+    cudaError_t e = device_alloc(ctx, (void**)&c->nodes, std::max<uint64_t>(h.node_words, 1) * 4);
+    if (e == cudaSuccess) e = device_alloc(ctx, (void**)&c->tapes, h.tape_words * 8);
     if (e == cudaSuccess) e = cudaMemcpy(c->nodes, p + blob_nodes_at(), h.node_words * 4, cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
         e = cudaMemcpy(c->tapes, p + blob_tapes_at(h.node_words), h.tape_words * 8, cudaMemcpyHostToDevice);

@@ -332,11 +332,11 @@ frep_status eval_common(frep_ctx* ctx, const void* code, uint64_t code_bytes, ui
                         const char* who) {
     const uint64_t tape_bytes = align_up(code_bytes + 8, 256);
     const uint64_t total = tape_bytes + align_up(in_bytes, 256) + align_up(slot_bytes, 256) + align_up(out_bytes, 256);
-    if (ctx->used + total > ctx->budget)
+    if (!frep::detail::reserve(ctx, total))
         return fail(FREP_ERR_OOM, "%s: %llu bytes of working memory exceed the context's budget", who,
                     (unsigned long long)total);
     FREP_CUDA(cudaSetDevice(ctx->device));
-    cudaError_t e = cudaMalloc(&buf->p, total);
+    cudaError_t e = frep::detail::device_alloc(ctx, &buf->p, total);
     if (e != cudaSuccess) {
         buf->p = nullptr;
         return fail(FREP_ERR_OOM, "%s: cudaMalloc of %llu bytes failed (%s)", who, (unsigned long long)total,

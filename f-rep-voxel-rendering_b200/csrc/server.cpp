@@ -574,13 +574,14 @@ frep_status frep_server_create(frep_ctx* ctx, const frep_server_config* config, 
     if (sv->cfg.max_batch > 65535) return fail(FREP_ERR_INVALID_ARG, "frep_server_create: max_batch above 65535");
     if (lights) sv->lights = *lights;
     else frep_lights_default(&sv->lights);
-    const uint64_t left = ctx->budget > ctx->used ? ctx->budget - ctx->used : 0;
+    const uint64_t left = frep::detail::budget_left(ctx);
     uint64_t arena = sv->cfg.hbm_budget ? sv->cfg.hbm_budget : left / 5 * 4;
     arena = align_up(arena, 4096);
-    if (arena == 0 || arena > left) return fail(FREP_ERR_OOM, "frep_server_create: arena of %llu bytes exceeds the budget",
-                                                (unsigned long long)arena);
+    if (arena == 0 || arena > left || !frep::detail::reserve(ctx, arena))
+        return fail(FREP_ERR_OOM, "frep_server_create: arena of %llu bytes exceeds the budget",
+                    (unsigned long long)arena);
     sv->cfg.hbm_budget = arena;
-    cudaError_t e = cudaMalloc(&sv->arena_mem, arena);
+    cudaError_t e = frep::detail::device_alloc(ctx, (void**)&sv->arena_mem, arena);
     if (e != cudaSuccess) return fail(FREP_ERR_OOM, "frep_server_create: cudaMalloc(%llu) failed (%s)",
                                       (unsigned long long)arena, cudaGetErrorString(e));
     sv->arena.reset(arena);
