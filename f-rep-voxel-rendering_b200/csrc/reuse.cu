@@ -27,6 +27,7 @@
 
 #include "device_common.cuh"
 #include "kernels.h"
+#include "micro_ops.h"
 
 namespace frep {
 namespace dev {
@@ -62,8 +63,10 @@ __device__ uint32_t prev_node_at(const TreeHeader* P, uint32_t L, uint32_t gx, u
     return pn;
 }
 
-// True when the tapes at a (pool A) and b (pool B) are identical and never
-// read slot 3 (the time) before writing it. Warp-uniform.
+// True when the tapes at a (pool A) and b (pool B) have the same instructions and
+// never read slot 3 (the time) before writing it. Their marks may differ (each
+// root tape had its own readers); either tape's hold for the words that it has.
+// Warp-uniform.
 __device__ bool same_time_free_tape(const uint64_t* A, uint32_t a, const uint64_t* B, uint32_t b, uint32_t lane) {
     const uint64_t ha = __ldcg(&A[a]), hb = __ldcg(&B[b]);
     if (ha != hb) return false;
@@ -74,7 +77,7 @@ __device__ bool same_time_free_tape(const uint64_t* A, uint32_t a, const uint64_
         const bool valid = i < n;
         const uint64_t wa = valid ? __ldcg(&A[a + 1 + i]) : 0ull;
         const uint64_t wb = valid ? __ldcg(&B[b + 1 + i]) : 0ull;
-        if (__any_sync(0xFFFFFFFFu, wa != wb)) return false;
+        if (__any_sync(0xFFFFFFFFu, ((wa ^ wb) & ~micro::MARKS) != 0ull)) return false;
         if (time_live) {
             const uint32_t op = w_op(wa);
             const bool reads = valid && op != OP_CONST && (w_a(wa) == 3u || (is_binary(op) && w_b(wa) == 3u));
