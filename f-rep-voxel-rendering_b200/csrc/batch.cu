@@ -48,7 +48,7 @@ struct frep_batch {
     frep_ctx* ctx = nullptr;
     std::vector<frep_tree*> trees;
     int rounding = 0;
-    // device work prefix (capacity + 1 entries) and cursor
+    // device work prefix (capacity + 1 entries), cursor and picked last-level pass
     unsigned long long* d_prefix = nullptr;
     unsigned long long* d_cursor = nullptr;
     uint32_t prefix_cap = 0;
@@ -172,7 +172,7 @@ frep_status ensure_prefix(frep_batch* b, uint32_t n) {
     // Growing waits for the device: start at 512 trees (a serving step's
     // default maximum) and double, so that a changing tree set rarely grows it.
     const uint32_t cap = std::max<uint32_t>(n, std::max<uint32_t>(512, 2 * b->prefix_cap));
-    FREP_CUDA(cudaMalloc(&b->d_prefix, sizeof(unsigned long long) * (cap + 2)));
+    FREP_CUDA(cudaMalloc(&b->d_prefix, sizeof(unsigned long long) * (cap + 3)));
     b->d_cursor = b->d_prefix + cap + 1;
     b->prefix_cap = cap;
     return FREP_OK;
@@ -207,6 +207,7 @@ frep_status ensure_keep(frep_batch* b, uint64_t words) {
 struct TapeStats {
     uint32_t slots = 4, mm = 1, longest = 1, max_levels = 0;
     uint64_t fine = 1;  // cells along an axis of the finest grid
+    double load[2][FREP_MAX_LEVELS] = {};  // leaf_load of the trees that end at a level (4, 2 cells per lane)
     bool any_k4 = false, any_k2 = false, pow2 = true;  // pow2: every last level's dim
 };
 
@@ -226,6 +227,7 @@ frep_status check_tapes(const frep_batch* b, const frep_tape* const* tapes, Tape
         st->fine = std::max(st->fine, frep::fine_cells(tr->grid.dims, tr->grid.levels));
         st->pow2 = st->pow2 && frep::pow2_dim(tr->grid.dims[tr->grid.levels - 1]);
         (tr->point_k == 4 ? st->any_k4 : st->any_k2) = true;
+        st->load[tr->point_k == 4 ? 0 : 1][tr->grid.levels - 1] += frep::leaf_load(tr->grid.dims, tr->grid.levels);
     }
     return FREP_OK;
 }
@@ -317,20 +319,26 @@ frep_status enqueue_voxelize(frep_batch* b, const uint8_t* d_area, const TapeSta
     a.n_slots = st.slots;
     a.mm_cap = st.mm;
     const int ki0 = level0_cells(b);
+    uint32_t launches = 1;
     for (uint32_t l = 0; l < st.max_levels; l++) {
         a.level = l;
         const int ki = l == 0 ? ki0 : b->plan4.interval_ki;
         e = frep::launch_level_scan(a, false, ki, s);
         if (e == cudaSuccess) e = frep::launch_level(a, b->plan4, b->rounding, false, s, ki);
         if (e != cudaSuccess) return cuda_fail(e, "batched interval pass");
+        launches += 2;
         if (prof) FREP_CUDA(cudaEventRecord(b->ev[2 + 3 * l], s));
         if (st.any_k4) {
+            a.leaf_load = st.load[0][l];
+            launches += frep::leaf_shape(a, b->plan4).blocks ? 3 : 2;
             e = frep::launch_level_scan(a, true, frep::leaf_items(a, b->plan4), s);
             if (e == cudaSuccess) e = frep::launch_level(a, b->plan4, b->rounding, true, s);
             if (e != cudaSuccess) return cuda_fail(e, "batched point pass");
         }
         if (prof) FREP_CUDA(cudaEventRecord(b->ev[3 + 3 * l], s));
         if (st.any_k2) {
+            a.leaf_load = st.load[1][l];
+            launches += frep::leaf_shape(a, b->plan2).blocks ? 3 : 2;
             e = frep::launch_level_scan(a, true, frep::leaf_items(a, b->plan2), s);
             if (e == cudaSuccess) e = frep::launch_level(a, b->plan2, b->rounding, true, s);
             if (e != cudaSuccess) return cuda_fail(e, "batched point pass");
@@ -341,7 +349,7 @@ frep_status enqueue_voxelize(frep_batch* b, const uint8_t* d_area, const TapeSta
         b->profiled = true;
         b->profiled_levels = st.max_levels;
     }
-    b->last_launches = 1 + 2 * st.max_levels * (1u + (st.any_k4 ? 1u : 0u) + (st.any_k2 ? 1u : 0u));
+    b->last_launches = launches;
     b->last_upload = L.total;
     return FREP_OK;
 }
@@ -610,6 +618,8 @@ frep_status frep_batch_run(frep_batch* b, const frep_tape* const* tapes, const f
                                  (uint64_t)b->plan4.leaf_blocks, (uint64_t)b->plan4.interval_ki,
                                  (uint64_t)level0_cells(b), (uint64_t)(uintptr_t)b->keep,
                                  (uint64_t)(uintptr_t)b->d_prefix, (uint64_t)(uintptr_t)A.d};
+    for (const auto& kind : st.load)  // (which launches leaf_shape gives a second pass)
+        for (const double load : kind) key.push_back((load > 0.0 ? 1u : 0u) + (load >= 1.0 ? 1u : 0u));
     for (uint32_t i = 0; i < n; i++) key.push_back(L.root_ofs[i]);
     if (!A.graph || key != A.graph_key) {
         if (A.graph) {

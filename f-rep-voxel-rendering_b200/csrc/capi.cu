@@ -374,7 +374,7 @@ frep_status tree_create_impl(frep_ctx* ctx, const frep_grid* grid, const frep_vo
     h.point_k = (uint32_t)t->point_k;
     t->d_self = reinterpret_cast<frep::dev::TreeHeader**>(t->d_small);
     t->d_prefix = t->d_small + 1;
-    t->d_cursor = t->d_small + 3;
+    t->d_cursor = t->d_small + 3;  // (and the picked pass after it)
     cudaError_t ce = cudaSuccess;
     if (ext) {  // written later by write_tree_header
         t->pending_hdr = h;
@@ -493,6 +493,7 @@ frep_status enqueue_tree_levels(frep_tree* tree, const frep_tape* tape, float ta
     a.n_trees = 1;
     a.keep_scratch = keep;
     a.longest = (uint32_t)tape->ct.instrs.size();
+    a.leaf_load = frep::leaf_load(g.dims, g.levels);
     a.keep_words = (uint64_t)plan.blocks * plan.warps_per_block * ws.stride;
     a.keep_stride = ws.stride;
     a.mm_ofs = ws.mm_ofs;

@@ -3,6 +3,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "leaf_rule.h"
+
 namespace frep {
 namespace dev {
 struct TreeHeader;
@@ -22,6 +24,7 @@ struct LevelLaunch {
     unsigned long long keep_words;     //   its size, u32 words (the last-level pass divides all of
                                        //   it among its warps)
     uint32_t longest;                  // instructions of the longest root tape
+    double leaf_load;                  // last-level pass: leaf_load of its trees, together
     uint32_t keep_stride;              //   u32 words per warp: keep masks [mm_ofs words,
     uint32_t mm_ofs;                   //   >= longest tape] then MIN/MAX choice masks
     uint32_t n_slots;                  // slot-file rows per lane (max over the batch)
@@ -35,6 +38,8 @@ struct LevelLaunch {
                                        //   kind (TreeHeader::point_k); 0: only trees of that kind
     uint32_t leaf_chunk;               // last-level pass: items per fetch at most, and a warp's share
     uint32_t leaf_share;               //   of the scratch in 8-byte words (set by launch_level)
+    uint32_t leaf_picked;              // 1: both last-level passes are launched and cursor[1] says
+                                       //   which of them runs (set by launch_level)
     uint32_t item_ofs;                 // per-warp scratch, u32 words: where the item tapes start
     uint32_t item_cap;                 //   and how many u64 words they may take (0 = no item
                                        //   pruning in the interval passes)
@@ -93,11 +98,12 @@ struct LevelPlan {
 // scratch of a few interval warps without item room holds fewer of those than
 // the pass has warps, and below half of them the point pass runs instead.
 struct LeafShape {
-    int blocks;      // 0: the point pass runs
+    int blocks;      // 0: the point pass alone is launched
     uint32_t share;  // 8-byte words of scratch per warp
 };
 inline LeafShape leaf_shape(const LevelLaunch& a, const LevelPlan& p) {
-    if (!p.leaf_warps_per_block) return LeafShape{0, 0u};
+    if (!p.leaf_warps_per_block || a.leaf_load == 0.0) return LeafShape{0, 0u};
+    if (a.leaf_load < 1.0 && a.longest < kLeafLongTape) return LeafShape{0, 0u};
     const uint64_t longest = (a.longest + 2ull) & ~1ull, words8 = a.keep_words / 2, w = (uint64_t)p.leaf_warps_per_block;
     uint64_t blocks = words8 / longest / w;
     if (blocks > (uint64_t)p.leaf_blocks) blocks = (uint64_t)p.leaf_blocks;
@@ -105,7 +111,8 @@ inline LeafShape leaf_shape(const LevelLaunch& a, const LevelPlan& p) {
     const uint64_t share = words8 / (blocks * w) & ~1ull;
     return LeafShape{(int)blocks, (uint32_t)(share < (1u << 24) ? share : 1u << 24)};
 }
-// `point_k` of launch_level_scan for a launch's last-level pass: its items.
+// `point_k` of launch_level_scan for a launch's last-level pass (negative: the
+// scan picks one of two passes).
 inline int leaf_items(const LevelLaunch& a, const LevelPlan& p) {
     return leaf_shape(a, p).blocks ? -p.point_k : p.point_k;
 }

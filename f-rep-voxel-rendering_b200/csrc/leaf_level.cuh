@@ -37,6 +37,12 @@ constexpr uint32_t LEAF_MIN_ROWS = LEAF_MAX_SLOTS * 128;  // bytes of the decode
 // Items per node of the pass, 8 mask words each (dim 4: the node's two).
 __host__ __device__ inline uint32_t leaf_units(uint32_t dim) { return dim == 4 ? 1u : (dim * dim * dim / 32u + 7u) / 8u; }
 
+// leaf_rule.h for a tree at its last level, in a launch of `cells` cells.
+__device__ __forceinline__ bool leaf_pays(const TreeHeader* H, uint32_t L, unsigned long long cells) {
+    return frep::leaf_pays(H->dims[L], H->transcendental != 0u, H->tape_size_sum[0],
+                           H->tape_size_sum[L] / max(1u, H->node_count[L]), cells);
+}
+
 #include "leaf_dispatch.cuh"
 
 // One micro-op that the loop leaves to C++, out of line, two cells at a time:
@@ -301,6 +307,7 @@ template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 5 : 20)
 leaf_level_kernel(LevelLaunch p) {
     extern __shared__ __align__(16) unsigned char smem[];
+    if (__ldcg(&p.cursor[1]) == 0ull) return;  // (point_level_kernel's launch)
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned char* wbase = smem + (size_t)warp * p.smem_per_warp;
     const uint32_t slot_bytes = p.smem_per_warp - LEAF_FIXED_BYTES;

@@ -849,8 +849,9 @@ __device__ __noinline__ uint32_t prepare_items(const uint64_t* tape, uint32_t n,
     // This evaluates and walks the node's tape once for the group, so a group of
     // one costs more than it saves (a level of 1,881 nodes with 849 words, of which
     // a warp fetches one item: 2.23 ms with, 1.40 without; 39 nodes with 526 words
-    // 296 and 140 us), as do tapes too short to lose much (19 words: 340 and 310 us).
-    if (g < 2u || n < 32u) return 0u;
+    // 296 and 140 us), as does a small group with a short tape (5 items, 19 words:
+    // 345 and 312 us; 30 items: 1.07 and 1.44 ms; 3 items, 62 words: 310 and 370 us).
+    if (g < 2u || g * n < 128u) return 0u;
     const uint32_t dim = T.dim, ncx = T.ncx, ncy = T.ncy, ncz = T.ncz;
     const bool valid = lane < g;
     // a tape with SIN / COS / EXP: the whole group runs the node's tape (found
@@ -1709,6 +1710,7 @@ template <int WARPS, int K>
 __global__ void __launch_bounds__(WARPS * 32)
 point_level_kernel(LevelLaunch p) {
     extern __shared__ __align__(16) unsigned char smem[];
+    if (p.leaf_picked && __ldcg(&p.cursor[1]) != 0ull) return;  // (leaf_level_kernel's launch)
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned char* wbase = smem + (size_t)warp * p.smem_per_warp;
     constexpr uint32_t ROW = 4 * K;  // bytes per lane per slot
@@ -1857,17 +1859,16 @@ point_level_kernel(LevelLaunch p) {
 // before i that this launch serves (interval passes: trees for which `level`
 // is not the last; point passes: trees for which it is, with a last-level node
 // size that takes `k` cells per lane). An item is k mask words of a node (k
-// cells per lane), or for k < 0 one of the leaf pass (trees of batch kind -k). Interval passes also fix where each tree's next level
-// starts (node_ofs[level + 1]). One block.
-__device__ __forceinline__ unsigned long long level_items(TreeHeader* H, uint32_t L, int point, int k,
+// cells per lane), or one of the leaf pass. Interval passes also fix where each
+// tree's next level starts (node_ofs[level + 1]). One block.
+__device__ __forceinline__ unsigned long long level_items(TreeHeader* H, uint32_t L, int point, int k, bool leaf,
                                                           bool write_ofs, bool reuse, bool any_k) {
     if (L >= H->levels) return 0;
     const bool last = L == H->levels - 1;
     if ((point != 0) != last) return 0;
     const uint32_t dim = H->dims[L];
     const uint32_t words = dim * dim * dim / 32;
-    const bool leaf = k < 0;
-    if (point && !any_k && H->point_k != (uint32_t)(leaf ? -k : k)) return 0;
+    if (point && !any_k && H->point_k != (uint32_t)k) return 0;
     const uint32_t count = level_count(H, L, H->node_cap, H->node_size[L]);
     if (!point && write_ofs) H->node_ofs[L + 1] = H->node_ofs[L] + (unsigned long long)count * H->node_size[L];
     // with reuse, only the listed nodes are evaluated
@@ -1882,8 +1883,32 @@ level_scan_kernel(TreeHeader* const* trees, uint32_t n, uint32_t L, int point, i
     const uint32_t t = threadIdx.x, T = blockDim.x;
     const uint32_t per = (n + T - 1) / T;
     const uint32_t b = min(n, t * per), e = min(n, b + per);
+    // point_k < 0: the last-level pass that more of the launch's cells vote for
+    // (leaf_pays), both being launched; the other finds cursor[1] against it.
+    __shared__ unsigned long long cells, votes;
+    bool leaf = false;
+    if (point_k < 0) {
+        point_k = -point_k;
+        if (t == 0) cells = votes = 0;
+        __syncthreads();
+        const auto cells_of = [&](uint32_t i) {  // (an item of point_k words: 32 point_k cells)
+            return level_items(trees[i], L, point, point_k, false, false, reuse != 0, any_k != 0) * (32u * (uint32_t)point_k);
+        };
+        unsigned long long mine = 0;
+        for (uint32_t i = b; i < e; i++) mine += cells_of(i);
+        if (mine) atomicAdd(&cells, mine);
+        __syncthreads();
+        mine = 0;
+        for (uint32_t i = b; i < e; i++) {
+            const unsigned long long c = cells_of(i);
+            if (c && leaf_pays(trees[i], L, cells)) mine += c;
+        }
+        if (mine) atomicAdd(&votes, mine);
+        __syncthreads();
+        leaf = 2 * votes > cells;
+    }
     unsigned long long sum = 0;
-    for (uint32_t i = b; i < e; i++) sum += level_items(trees[i], L, point, point_k, true, reuse != 0, any_k != 0);
+    for (uint32_t i = b; i < e; i++) sum += level_items(trees[i], L, point, point_k, leaf, true, reuse != 0, any_k != 0);
     part[t] = sum;
     __syncthreads();
     for (uint32_t off = 1; off < T; off <<= 1) {  // inclusive scan
@@ -1895,10 +1920,13 @@ level_scan_kernel(TreeHeader* const* trees, uint32_t n, uint32_t L, int point, i
     unsigned long long run = part[t] - sum;
     for (uint32_t i = b; i < e; i++) {
         prefix[i] = run;
-        run += level_items(trees[i], L, point, point_k, false, reuse != 0, any_k != 0);
+        run += level_items(trees[i], L, point, point_k, leaf, false, reuse != 0, any_k != 0);
     }
     if (t == T - 1) prefix[n] = part[t];
-    if (t == 0) *cursor = 0ull;
+    if (t == 0) {
+        cursor[0] = 0ull;
+        cursor[1] = leaf ? 1ull : 0ull;
+    }
 }
 
 // A root at an interval level (more than one level) starts with zeroed mask
@@ -2167,7 +2195,9 @@ cudaError_t launch_tree_init_staged(dev::TreeHeader* const* trees, uint32_t n, c
 }
 
 cudaError_t launch_level_scan(const LevelLaunch& a, bool point, int point_k, cudaStream_t stream) {
-    dev::level_scan_kernel<<<1, 1024, 0, stream>>>(a.trees, a.n_trees, a.level, point ? 1 : 0, point_k, a.prefix,
+    // (a warp for one tree: 3 us, 4.4 with 1,024 threads)
+    const uint32_t threads = a.n_trees < 1024 ? (a.n_trees + 31) / 32 * 32 : 1024;
+    dev::level_scan_kernel<<<1, threads, 0, stream>>>(a.trees, a.n_trees, a.level, point ? 1 : 0, point_k, a.prefix,
                                                    a.cursor, a.eval_list ? 1 : 0, a.any_point_k ? 1 : 0);
     return cudaGetLastError();
 }
@@ -2189,10 +2219,12 @@ cudaError_t launch_level(const LevelLaunch& a, const LevelPlan& plan, int roundi
         const size_t smem = (size_t)w * plan.leaf_smem_per_warp;
         if (w == 4) dev::leaf_level_kernel<4><<<leaf.blocks, 128, smem, stream>>>(b);
         else dev::leaf_level_kernel<1><<<leaf.blocks, 32, smem, stream>>>(b);
-        return cudaGetLastError();
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
     }
     if (point) {
         LevelLaunch b = a;
+        b.leaf_picked = leaf.blocks ? 1u : 0u;
         b.smem_per_warp = plan.point_smem_per_warp;
         const int w4 = plan.point_warps_per_block == 4;
         const size_t smem = (size_t)plan.point_warps_per_block * plan.point_smem_per_warp;
