@@ -587,7 +587,7 @@ typedef struct frep_autotune_opts {
     uint32_t reps;           /* timed runs per candidate; the median counts (0 = 5)        */
     uint32_t width, height;  /* frame size of the timed renders (0 = 512 x 512)            */
     float margin;            /* a candidate replaces the incumbent only when faster by this
-                              * fraction (0 = 0.03)                                        */
+                              * fraction (0 = 0.03), a cached choice when by twice of it   */
     uint32_t force;          /* 1: tune every class afresh, cached choices ignored         */
     uint32_t refine;         /* 1: re-time cached classes too, the cached choice first      */
 } frep_autotune_opts;
@@ -599,8 +599,8 @@ typedef struct frep_autotune_opts {
  * render of up to per_class scenes of the class under CUDA graph replay (the
  * median of reps runs); then the tapes per block on up to 32 scenes spread
  * over the batch. The incumbent of a class (its cached choice, else the
- * first candidate) is kept unless a candidate beats it by `margin`, so a
- * repeated tuning keeps its choices. Classes already in `tuning` are skipped
+ * first candidate) is kept unless a candidate beats it by `margin` (a cached
+ * choice: by 2 `margin`), so a repeated tuning keeps its choices. Classes already in `tuning` are skipped
  * unless force or refine. Blocking; allocates and frees its own trees. */
 frep_status frep_batch_autotune(frep_ctx* ctx, const frep_tape* const* tapes, const uint32_t* resolutions,
                                 const frep_camera* cameras, uint32_t n, const frep_lights* lights,
