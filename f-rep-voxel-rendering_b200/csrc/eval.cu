@@ -238,20 +238,24 @@ struct PointCode {
     uint32_t rows = 4, result = 0;  // rows of the slot file, offset of the result's
 };
 
+// Stops, with rows above EVAL_MAX_ROWS, at the record that would need as many.
 PointCode point_code(const std::vector<uint64_t>& instrs, uint32_t n_slots) {
     constexpr uint32_t T = frep::dev::EVAL_THREADS, CONST = ~0u, INPUTS = 4;
     struct Ref {
         uint32_t value = CONST, bits = 0;  // a value's number, or a constant
     };
     struct Value {
-        uint32_t op = 0, need = 0, last = 0;
+        uint32_t op = 0, need = 0, uses = 0, row = 0;
         Ref a, b;
         bool placed = false;
     };
-    std::vector<Value> v(INPUTS);
+    std::vector<Value> v;
+    v.reserve(INPUTS + instrs.size() + 1);
+    v.resize(INPUTS);
     std::vector<Ref> slot(n_slots);
     for (uint32_t i = 0; i < INPUTS; i++) {
         slot[i].value = i;
+        v[i].row = i;
         v[i].placed = true;
     }
     for (const uint64_t w : instrs) {
@@ -276,53 +280,54 @@ PointCode point_code(const std::vector<uint64_t>& instrs, uint32_t n_slots) {
         slot[0] = Ref{(uint32_t)v.size(), 0};
         v.push_back(x);
     }
-    // Depth first from the result.
+    // How often the result's values are used (operands come before their user).
     const uint32_t result = slot[0].value;
-    std::vector<uint32_t> order, stack = {result};
+    for (uint32_t i = result; i >= INPUTS; i--) {
+        if (i != result && v[i].uses == 0) continue;
+        for (const uint32_t u : {v[i].a.value, v[i].b.value})
+            if (u != CONST) v[u].uses++;
+    }
+    // Depth first from the result.
+    PointCode code;
+    code.recs.reserve(v.size());
+    std::vector<uint32_t> stack = {result}, free_rows;
     while (!stack.empty()) {
         const uint32_t i = stack.back();
-        if (v[i].placed) {
+        Value& x = v[i];
+        if (x.placed) {
             stack.pop_back();
             continue;
         }
-        const uint32_t a = v[i].a.value, b = v[i].b.value;
+        const uint32_t a = x.a.value, b = x.b.value;
         const bool wait_a = a != CONST && !v[a].placed, wait_b = b != CONST && !v[b].placed;
-        if (!wait_a && !wait_b) {
-            v[i].placed = true;
-            for (const uint32_t u : {a, b})
-                if (u != CONST) v[u].last = (uint32_t)order.size();
-            order.push_back(i);
-            stack.pop_back();
-        } else {  // the top of the stack is placed first
+        if (wait_a || wait_b) {  // the top of the stack is placed first
             const bool a_first = wait_a && (!wait_b || v[a].need >= v[b].need);
             if (a_first && wait_b) stack.push_back(b);
             if (wait_a) stack.push_back(a);
             if (!a_first && wait_b) stack.push_back(b);
+            continue;
         }
-    }
-    PointCode code;
-    std::vector<uint32_t> row(v.size(), 0), free_rows;
-    for (uint32_t i = 0; i < INPUTS; i++) row[i] = i;
-    for (uint32_t at = 0; at < order.size(); at++) {
-        const Value& x = v[order[at]];
+        stack.pop_back();
+        x.placed = true;
         uint4 q = make_uint4(x.a.bits, x.b.bits, 0, x.op);
-        if (x.a.value == CONST) q.w |= frep::dev::EVAL_IMM_A;
-        else q.x = row[x.a.value] * T;
+        if (a == CONST) q.w |= frep::dev::EVAL_IMM_A;
+        else q.x = v[a].row * T;
         if (!frep::dev::is_binary(x.op)) q.y = 0;
-        else if (x.b.value == CONST) q.w |= frep::dev::EVAL_IMM_B;
-        else q.y = row[x.b.value] * T;
-        for (const uint32_t u : {x.a.value, x.b.value == x.a.value ? CONST : x.b.value})
-            if (u != CONST && u >= INPUTS && v[u].last == at) free_rows.push_back(row[u]);
+        else if (b == CONST) q.w |= frep::dev::EVAL_IMM_B;
+        else q.y = v[b].row * T;
+        for (const uint32_t u : {a, b})
+            if (u != CONST && --v[u].uses == 0 && u >= INPUTS) free_rows.push_back(v[u].row);
         if (free_rows.empty()) {
-            row[order[at]] = code.rows++;
+            x.row = code.rows++;
+            if (code.rows > frep::dev::EVAL_MAX_ROWS) return code;
         } else {
-            row[order[at]] = free_rows.back();
+            x.row = free_rows.back();
             free_rows.pop_back();
         }
-        q.z = row[order[at]] * T;
+        q.z = x.row * T;
         code.recs.push_back(q);
     }
-    code.result = row[result] * T;
+    code.result = v[result].row * T;
     return code;
 }
 
@@ -367,7 +372,7 @@ extern "C" frep_status frep_tape_eval_device(frep_ctx* ctx, const frep_tape* tap
     if (st != FREP_OK) return st;
     const PointCode pc = point_code(tape->ct.instrs, n_slots);
     const bool shared = pc.rows <= frep::dev::EVAL_MAX_ROWS;
-    const uint32_t K = n >= 148u * 2 * T * 4 ? 4 : 1;
+    const uint32_t K = n >= (uint64_t)ctx->sm_count * 2 * T * 4 ? 4 : 1;
     EvalBuffers buf;
     uint8_t *d_in, *d_slots, *d_out;
     const void* code = shared ? static_cast<const void*>(pc.recs.data()) : tape->ct.instrs.data();
