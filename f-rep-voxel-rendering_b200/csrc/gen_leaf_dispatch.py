@@ -27,7 +27,7 @@ OPS = {"CONST": 0, "SIN": 1, "COS": 2, "ADD": 3, "SUB": 4, "MUL": 5, "DIV": 6, "
        "EXP": 9, "NEG": 10, "SQRT": 11, "COPY": 12, "END": 13}
 KINDS = "SFI"  # operand kinds: slot row, forwarded, constant
 SOURCES = ["SS", "FS", "SF", "FF", "SI", "FI", "IS", "IF"]
-COMMUTATIVE = ("ADD", "MUL")  # make_micro puts F before S and I last
+COMMUTATIVE = ("ADD", "MUL")  # decode_word and decode_single put F before S and I last
 BINARY = ("ADD", "SUB", "MUL", "MIN", "MAX")
 UNARY = ("NEG", "COPY", "SQRT")
 TABLE = 2 * 256

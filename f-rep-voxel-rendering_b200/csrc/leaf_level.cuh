@@ -220,7 +220,7 @@ __device__ __forceinline__ void leaf_run(const LevelTree& T, const LeafTape& tp,
                                          uint32_t lane,
                                          const float (&nx)[K / 2], const float (&ny)[K / 2], const float (&nz)[K / 2],
                                          const uint32_t (&wd)[K], uint32_t (&leaf)[K]) {
-    const uint32_t lane_base = slot_base + lane * (K == 8 ? 16u : 4u * K);
+    const uint32_t lane_base = slot_base + lane * (4u * K);
     // (voxelizer/main.comp:74-79; the sums are whole numbers below 2^24, exact)
     FK<K> px, py, pz;
 #pragma unroll

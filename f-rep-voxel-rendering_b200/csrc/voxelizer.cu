@@ -518,22 +518,18 @@ __device__ __forceinline__ void walk_lanes(const uint64_t* tape, uint32_t n, int
 }
 
 // The same for a warp that has an SM (nearly) to itself, a single tree's root
-// level: the serial chain per instruction is one shuffle and the updates after
-// it, dead instructions go through it without a branch, and the next word is
-// fetched one instruction early (75 primitives: root level 0.69 -> 0.54 ms). Its
-// two loop bodies cost the levels below, with 16 warps per SM and more code
-// beside, more than they save (a batch's level 1 27.0 -> 29.1 ms).
-template <int KI, int S>
+// level with one cell per lane and at most 32 slots: the serial chain per
+// instruction is one shuffle and the updates after it, dead instructions go
+// through it without a branch, and the next word is fetched one instruction early
+// (75 primitives: root level 0.69 -> 0.54 ms). Its two loop bodies cost the levels
+// below, with 16 warps per SM and more code beside, more than they save (a batch's
+// level 1 27.0 -> 29.1 ms).
 __device__ __forceinline__ void walk_lanes_alone(const uint64_t* tape, uint32_t n, int mm, const uint2* mmb,
-                                           uint32_t* keep, const uint32_t (&ok_w)[KI], uint32_t lane,
-                                           uint32_t (&kept)[KI], uint32_t (&sig)[KI]) {
-    uint32_t lv[S][KI];
-#pragma unroll
-    for (int q = 0; q < S; q++)
-#pragma unroll
-        for (int h = 0; h < KI; h++) lv[q][h] = (q == 0 && lane == 0) ? ok_w[h] : 0u;  // slot 0: the result
-    bool plain = true;  // (the top chunk: mostly live)
-    int mm_top = mm;    // MIN/MAX instructions before the current chunk's end
+                                                 uint32_t* keep, uint32_t ok_w, uint32_t lane, uint32_t& kept,
+                                                 uint32_t& sig) {
+    uint32_t lv = lane == 0 ? ok_w : 0u;  // lane l: slot l; slot 0: the result
+    bool plain = true;                    // (the top chunk: mostly live)
+    int mm_top = mm;                      // MIN/MAX instructions before the current chunk's end
     for (int hi = (int)n; hi > 0; hi -= 32) {
         const int lo = max(0, hi - 32);
         const int m = hi - lo;
@@ -546,53 +542,27 @@ __device__ __forceinline__ void walk_lanes_alone(const uint64_t* tape, uint32_t 
                             (mop != OP_CONST ? 1u << 18 : 0u) | (is_binary(mop) ? 1u << 19 : 0u) | (ism ? 1u << 20 : 0u);
         const uint32_t mball = __ballot_sync(0xFFFFFFFFu, ism);
         const int mbase = mm_top - __popc(mball);
-        uint2 cb[KI];
-#pragma unroll
-        for (int h = 0; h < KI; h++)
-            cb[h] = ism ? mmb[(mbase + __popc(mball & lanemask_lt())) * KI + h] : make_uint2(0u, 0u);
-        uint32_t my_keep[KI], my_f[KI], my_s[KI];  // this lane's instruction: keep / chosen-input masks
-#pragma unroll
-        for (int h = 0; h < KI; h++) my_keep[h] = my_f[h] = my_s[h] = 0u;
+        const uint2 cb = ism ? mmb[mbase + __popc(mball & lanemask_lt())] : make_uint2(0u, 0u);
+        uint32_t my_keep = 0u, my_f = 0u, my_s = 0u;  // this lane's instruction: keep / chosen-input masks
         int live = 0;  // instructions of this chunk live in some cell
         int j = m - 1;
         // instruction j (q: its packed word), live or not
         auto step = [&](uint32_t q) {
             const uint32_t o = q & 63u, a = (q >> 6) & 63u, b = (q >> 12) & 63u;
-            uint32_t k[KI], f[KI], sc[KI], anyk = 0;
-#pragma unroll
-            for (int h = 0; h < KI; h++) {
-                const uint32_t src = (S == 2 && o >= 32u) ? lv[S - 1][h] : lv[0][h];
-                k[h] = __shfl_sync(0xFFFFFFFFu, src, o & 31u);
-                anyk |= k[h];
-                f[h] = (q >> 18) & 1u ? k[h] : 0u;
-                sc[h] = (q >> 19) & 1u ? k[h] : 0u;
-            }
+            const uint32_t k = __shfl_sync(0xFFFFFFFFu, lv, o & 31u);
+            uint32_t f = (q >> 18) & 1u ? k : 0u, sc = (q >> 19) & 1u ? k : 0u;
             if ((q >> 20) & 1u) {
-#pragma unroll
-                for (int h = 0; h < KI; h++) {
-                    f[h] &= __shfl_sync(0xFFFFFFFFu, cb[h].x, j);
-                    sc[h] &= __shfl_sync(0xFFFFFFFFu, cb[h].y, j);
-                    if ((int)lane == j) {
-                        my_f[h] = f[h];
-                        my_s[h] = sc[h];
-                    }
+                f &= __shfl_sync(0xFFFFFFFFu, cb.x, j);
+                sc &= __shfl_sync(0xFFFFFFFFu, cb.y, j);
+                if ((int)lane == j) {
+                    my_f = f;
+                    my_s = sc;
                 }
             }
-            live += anyk != 0u;
+            live += k != 0u;
             // clear the output slot, then set the inputs the choice uses
-            const bool at_o = lane == (o & 31u), at_a = lane == (a & 31u), at_b = lane == (b & 31u);
-#pragma unroll
-            for (int h = 0; h < KI; h++) {
-                if constexpr (S == 1) {
-                    lv[0][h] = (at_o ? 0u : lv[0][h]) | (at_a ? f[h] : 0u) | (at_b ? sc[h] : 0u);
-                } else {
-                    lv[0][h] = (at_o && o < 32u ? 0u : lv[0][h]) | (at_a && a < 32u ? f[h] : 0u) |
-                               (at_b && b < 32u ? sc[h] : 0u);
-                    lv[S - 1][h] = (at_o && o >= 32u ? 0u : lv[S - 1][h]) | (at_a && a >= 32u ? f[h] : 0u) |
-                                   (at_b && b >= 32u ? sc[h] : 0u);
-                }
-                if ((int)lane == j) my_keep[h] = k[h];
-            }
+            lv = (lane == (o & 31u) ? 0u : lv) | (lane == (a & 31u) ? f : 0u) | (lane == (b & 31u) ? sc : 0u);
+            if ((int)lane == j) my_keep = k;
         };
         if (plain) {
             uint32_t q = __shfl_sync(0xFFFFFFFFu, pk, j);
@@ -604,15 +574,8 @@ __device__ __forceinline__ void walk_lanes_alone(const uint64_t* tape, uint32_t 
             }
         } else {
             while (j >= 0) {
-                uint32_t u0 = 0, u1 = 0;
-#pragma unroll
-                for (int h = 0; h < KI; h++) {
-                    u0 |= lv[0][h];
-                    if constexpr (S == 2) u1 |= lv[S - 1][h];
-                }
-                const uint64_t U = (uint64_t)__ballot_sync(0xFFFFFFFFu, u0 != 0u) |
-                                   (S == 2 ? (uint64_t)__ballot_sync(0xFFFFFFFFu, u1 != 0u) << 32 : 0ull);
-                const uint32_t cand = __ballot_sync(0xFFFFFFFFu, (int)lane <= j && ((U >> (pk & 63u)) & 1ull));
+                const uint32_t U = __ballot_sync(0xFFFFFFFFu, lv != 0u);
+                const uint32_t cand = __ballot_sync(0xFFFFFFFFu, (int)lane <= j && ((U >> (pk & 31u)) & 1u));
                 if (!cand) break;
                 j = 31 - __clz(cand);
                 step(__shfl_sync(0xFFFFFFFFu, pk, j));
@@ -620,22 +583,17 @@ __device__ __forceinline__ void walk_lanes_alone(const uint64_t* tape, uint32_t 
             }
         }
         plain = 2 * live >= m;  // the next chunk's mode, from this one's liveness
-        if ((int)lane < m) {
-            if constexpr (KI == 1) keep[lo + lane] = my_keep[0];
-            else reinterpret_cast<uint2*>(keep)[lo + lane] = make_uint2(my_keep[0], my_keep[1]);
-        }
+        if ((int)lane < m) keep[lo + lane] = my_keep;
         // per cell: the chunk's kept instructions and MIN/MAX rewrites
-#pragma unroll
-        for (int h = 0; h < KI; h++) {
-            if (!__any_sync(0xFFFFFFFFu, my_keep[h] != 0u)) continue;
-            const uint32_t kc = transpose32(my_keep[h], lane);
-            kept[h] += __popc(kc);
+        if (__any_sync(0xFFFFFFFFu, my_keep != 0u)) {
+            const uint32_t kc = transpose32(my_keep, lane);
+            kept += __popc(kc);
             uint32_t fc = 0, sc = 0;
-            if (__any_sync(0xFFFFFFFFu, (my_f[h] | my_s[h]) != 0u)) {
-                fc = transpose32(my_f[h], lane);
-                sc = transpose32(my_s[h], lane);
+            if (__any_sync(0xFFFFFFFFu, (my_f | my_s) != 0u)) {
+                fc = transpose32(my_f, lane);
+                sc = transpose32(my_s, lane);
             }
-            sig[h] = sig[h] * 0x9E3779B1u + (kc ^ (uint32_t)lo) * 0x85EBCA6Bu + fc * 0xC2B2AE35u + sc * 0x27D4EB2Fu;
+            sig = sig * 0x9E3779B1u + (kc ^ (uint32_t)lo) * 0x85EBCA6Bu + fc * 0xC2B2AE35u + sc * 0x27D4EB2Fu;
         }
         mm_top = mbase;
     }
@@ -1310,7 +1268,7 @@ interval_level_kernel(LevelLaunch p) {
                 if (p.n_slots <= 32) {
                     // live sets spread over the lanes' registers: no shared
                     // memory on the walk's path
-                    if constexpr (MO && KI == 1) walk_lanes_alone<1, 1>(tape, n, (int)mm, mmb, keep, ok_w, lane, kept, sig);
+                    if constexpr (MO && KI == 1) walk_lanes_alone(tape, n, (int)mm, mmb, keep, ok_w[0], lane, kept[0], sig[0]);
                     else walk_lanes<KI, 1>(tape, n, (int)mm, mmb, keep, ok_w, lane, kept, sig);
                 } else if (p.n_slots <= 64) {
                     walk_lanes<KI, 2>(tape, n, (int)mm, mmb, keep, ok_w, lane, kept, sig);
