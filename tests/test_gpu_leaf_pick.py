@@ -85,6 +85,23 @@ def test_reuse_lists_nodes_for_either_pass(ctx):
         t.cleanup()
 
 
+@pytest.mark.parametrize("rounding", [1, 2])
+def test_scratch_of_fitted_pools(ctx, rounding):
+    """Trees whose pools leave no item room: the pass over micro-ops gets what the
+    interval passes' masks take (one cell per lane from 24 slots on and in the
+    hybrid mode), all, half or too little of its warps."""
+    from frep.autotune import fit_pools
+    for shape in (CSG, scenes.spheres_union(22).shape, scenes.spheres_union(30).shape,
+                  scenes.random_csg(33, seed=33).shape, scenes.MengerSponge(2)):
+        sc = _scene(shape, [16, 16, 4])
+        p = fit_pools(ctx, [sc.shape], [sc.grid_dims], sc.low_vertex, sc.world_size, margin=0.25)[0]
+        vs = frep.VoxelStorage(sc.grid_dims, sc.low_vertex, sc.world_size, rounding=rounding, node_words=p.node_words,
+                               tape_words=p.tape_words).init(ctx, sc.shape)
+        frep.Voxelizer(ctx, vs).voxelize(0.0)
+        assert compare_trees_fast(vs.export(), oracle_tree(sc, vs.tape, rounding=rounding)) == [], vs.tape.n_slots
+        vs.cleanup()
+
+
 def test_batches(ctx):
     """Twelve trees are together what one of them is not; the trees of a batch
     keep one pass per last dim class, whatever else ends at that level."""
