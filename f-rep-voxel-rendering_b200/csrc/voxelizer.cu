@@ -940,6 +940,7 @@ template <int ROUND, int WARPS, int KI, bool MO>
 // Shared memory already limits a batch's plan to about 16 resident warps, and
 // a cap of 96 registers spills inside the forward pass: on a 128-scene batch
 // the level-1 pass measured 35.0 ms with the cap and 26.7 ms without.
+// (At 128 the instances for two cells still spill 180 bytes, the root's 316.)
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 4 : 16)
 interval_level_kernel(LevelLaunch p) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -2058,9 +2059,11 @@ static cudaError_t plan_point(uint32_t n_slots, LevelPlan* plan, int warps_hint)
     return occupancy(dev::point_level_kernel<1, K>, 32, pt, &plan->point_blocks);
 }
 
-// The last-level pass over micro-ops takes every tape whose slots fit the row
-// mask, on grids whose last dims are powers of two and cell numbers exact floats. Rows for a warp: 20 warps to an SM (14 rows of 4 cells per lane, 28 of
-// 2), or what 2 cells per lane need for every slot of the batch.
+// The last-level pass over micro-ops can take every tape whose slots fit the row
+// mask, on grids whose last dims are powers of two and cell numbers exact floats
+// (leaf_rule.h: when it does). Rows for a warp: 20 warps to an SM (14 rows of 4
+// cells per lane, 28 of 2), or what 2 cells per lane need for every slot of the
+// batch.
 static cudaError_t plan_leaf(uint32_t n_slots, LevelPlan* plan, int warps_hint) {
     static_assert(kLeafSlotBytes >= dev::LEAF_MIN_ROWS && kLeafSlotBytes % 16 == 0, "the decoder's constants fit");
     const uint32_t rows = std::max<uint32_t>(kLeafSlotBytes, n_slots * 256);
