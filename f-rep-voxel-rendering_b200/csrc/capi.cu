@@ -475,9 +475,10 @@ frep_status ensure_plan(frep_tree* tree, const frep_tape* tape, const char* who)
 // With `prev`, nodes whose time-free tape equals prev's at the same place are
 // copied from it (reuse.cu): a match pass fixes every node's source before its
 // level pass, and a copy pass follows it.
+// keep: the scratch, of keep_words words.
 frep_status enqueue_tree_levels(frep_tree* tree, const frep_tape* tape, float tape_time, uint32_t* keep,
-                                frep::WarpScratch ws, const frep::LevelPlan& plan, cudaStream_t stream,
-                                const frep_tree* prev = nullptr) {
+                                uint64_t keep_words, frep::WarpScratch ws, const frep::LevelPlan& plan,
+                                cudaStream_t stream, const frep_tree* prev = nullptr) {
     cudaError_t e = frep::launch_tree_init(tree->d_self, 1, nullptr, tape_time, tape->transcendental, stream);
     if (e != cudaSuccess) return cuda_fail(e, "tree_init_kernel");
     if (prev) {
@@ -494,7 +495,7 @@ frep_status enqueue_tree_levels(frep_tree* tree, const frep_tape* tape, float ta
     a.keep_scratch = keep;
     a.longest = (uint32_t)tape->ct.instrs.size();
     a.leaf_load = frep::leaf_load(g.dims, g.levels);
-    a.keep_words = (uint64_t)plan.blocks * plan.warps_per_block * ws.stride;
+    a.keep_words = keep_words;
     a.keep_stride = ws.stride;
     a.mm_ofs = ws.mm_ofs;
     a.item_ofs = ws.item_ofs;
@@ -611,6 +612,17 @@ frep_status voxelize_impl(frep_ctx* ctx, frep_tree* tree, const frep_tree* prev,
     }
     const uint64_t need = warps * plain.stride;
     uint64_t keep_words = warps * ws.stride;
+    // The last-level pass over micro-ops wants a record of the root tape's length
+    // for each of its warps. Masks for two cells per lane hold about that; for one
+    // (24 slots and more, the hybrid mode) half of it or less, and the pass was
+    // lost for a few MB (22 spheres, 547,000 dim-4 nodes: 0.56 ms, 0.28 with the
+    // room). The same bounds as item room.
+    if (tree->prune_items && frep::leaf_wanted(frep::leaf_load(tree->grid.dims, tree->grid.levels), n, tree->plan)) {
+        const uint64_t leaf = (uint64_t)tree->plan.leaf_blocks * tree->plan.leaf_warps_per_block * frep::leaf_record(n) * 2;
+        const uint64_t most = std::min((tree->node_cap * 4 + tree->tape_cap * 8) / 4, warps * frep::kTreeItemTapeWords * 8);
+        if (leaf > keep_words && (leaf - need) * 4 <= most && (leaf <= tree->keep_words || others + leaf * 4 <= ctx->budget))
+            keep_words = leaf;
+    }
     if (keep_words > tree->keep_words) {
         // (a tree that sees ever longer tapes, as when pools are fitted, grows it
         // by half at least, within the budget: each growth waits for the stream)
@@ -669,7 +681,7 @@ frep_status voxelize_impl(frep_ctx* ctx, frep_tree* tree, const frep_tree* prev,
     tree->root_words = (uint32_t)root_words;
     tree->stream = stream;
 
-    return enqueue_tree_levels(tree, tape, tape_time, tree->keep, ws, tree->plan, stream, prev);
+    return enqueue_tree_levels(tree, tape, tape_time, tree->keep, tree->keep_words, ws, tree->plan, stream, prev);
 }
 
 }  // namespace
@@ -1021,5 +1033,5 @@ extern "C" frep_status frep_voxelize_static_scratch(frep_ctx* ctx, frep_tree* tr
     tree->root_words = (uint32_t)root_words;
     tree->stream = stream;
 
-    return enqueue_tree_levels(tree, tape, tape_time, scratch, ws, plan, stream);
+    return enqueue_tree_levels(tree, tape, tape_time, scratch, (uint64_t)plan.blocks * per_block, ws, plan, stream);
 }

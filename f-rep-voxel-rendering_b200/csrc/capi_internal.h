@@ -99,7 +99,7 @@ struct frep_tree {
     frep_voxelize_opts opts{};
     int point_k = 4;  // cells per lane of the last-level pass in batches (its batch kind, 4 or 2)
     int plain_k = 4;  // cells per lane of its own last-level passes (frep_voxelize and variants)
-    bool prune_items = true;  // its own passes may take room for item tapes
+    bool prune_items = true;  // its own passes may take room (item tapes, micro-ops)
     bool external = false;  // header and pools live in caller-owned memory
     bool hdr_pending = false;              // external: header not yet written to the device
     frep::dev::TreeHeader pending_hdr{};   //   (write_tree_header)

@@ -94,17 +94,21 @@ struct LevelPlan {
     uint32_t leaf_smem_per_warp;
 };
 // How the last-level pass over micro-ops runs a launch. A warp's share of the
-// scratch holds the micro-ops of the longest tape (at most one per word); the
-// scratch of a few interval warps without item room holds fewer of those than
-// the pass has warps, and below half of them the point pass runs instead.
+// scratch holds the micro-ops of the longest tape (at most one per word); scratch
+// without room (item tapes', or what frep_voxelize adds for this pass) holds fewer
+// of those than the pass has warps, and below half of them the point pass runs
+// instead.
 struct LeafShape {
     int blocks;      // 0: the point pass alone is launched
     uint32_t share;  // 8-byte words of scratch per warp
 };
+inline bool leaf_wanted(double load, uint32_t longest, const LevelPlan& p) {
+    return p.leaf_warps_per_block && load != 0.0 && (load >= 1.0 || longest >= kLeafLongTape);
+}
+inline uint64_t leaf_record(uint32_t longest) { return (longest + 2ull) & ~1ull; }  // 8-byte words
 inline LeafShape leaf_shape(const LevelLaunch& a, const LevelPlan& p) {
-    if (!p.leaf_warps_per_block || a.leaf_load == 0.0) return LeafShape{0, 0u};
-    if (a.leaf_load < 1.0 && a.longest < kLeafLongTape) return LeafShape{0, 0u};
-    const uint64_t longest = (a.longest + 2ull) & ~1ull, words8 = a.keep_words / 2, w = (uint64_t)p.leaf_warps_per_block;
+    if (!leaf_wanted(a.leaf_load, a.longest, p)) return LeafShape{0, 0u};
+    const uint64_t longest = leaf_record(a.longest), words8 = a.keep_words / 2, w = (uint64_t)p.leaf_warps_per_block;
     uint64_t blocks = words8 / longest / w;
     if (blocks > (uint64_t)p.leaf_blocks) blocks = (uint64_t)p.leaf_blocks;
     if (2 * blocks < (uint64_t)p.leaf_blocks) return LeafShape{0, 0u};

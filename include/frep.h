@@ -206,8 +206,9 @@ typedef struct frep_tree frep_tree;
  * from the context's budget). The tree can be re-voxelized many times.
  * Its first voxelization by frep_voxelize or frep_voxelize_reuse allocates
  * scratch from the budget, which it keeps and grows for longer tapes: masks for
- * every instruction and, where the budget holds it, at most a quarter of the
- * pools' bytes (80 MB at most) and half again on growth. This second part makes
+ * every instruction and, where the budget holds it, room for shortened and
+ * decoded tapes of at most a quarter of the pools' bytes (80 MB at most) and half
+ * again on growth. This second part makes
  * level passes faster and gives way: an allocation of the context that the
  * budget would refuse takes it back first (and waits for the device), except
  * from trees whose voxelization was captured in a graph. */

@@ -102,6 +102,22 @@ def test_scratch_of_fitted_pools(ctx, rounding):
         vs.cleanup()
 
 
+def test_fitted_pools_leave_room_for_one_cell_plans(ctx):
+    """25 slots: the interval passes run one cell per lane and their masks hold
+    less than half of a record for each warp of the pass over micro-ops."""
+    from frep.autotune import fit_pools
+    sc = _scene(scenes.spheres_union(22).shape, [32, 16, 4])
+    p = fit_pools(ctx, [sc.shape], [sc.grid_dims], sc.low_vertex, sc.world_size, margin=0.25)[0]
+    vs = frep.VoxelStorage(sc.grid_dims, sc.low_vertex, sc.world_size, node_words=p.node_words,
+                           tape_words=p.tape_words).init(ctx, sc.shape)
+    v = frep.Voxelizer(ctx, vs)
+    v.voxelize(0.0)
+    assert compare_trees_fast(vs.export(), oracle_tree(sc, vs.tape)) == []
+    ops, words = _passes(lambda: v.voxelize(0.0))
+    assert ops > words, (ops, words)
+    vs.cleanup()
+
+
 def test_batches(ctx):
     """Twelve trees are together what one of them is not; the trees of a batch
     keep one pass per last dim class, whatever else ends at that level."""
