@@ -208,10 +208,10 @@ typedef struct frep_tree frep_tree;
  * scratch from the budget, which it keeps and grows for longer tapes: masks for
  * every instruction and, where the budget holds it, room for shortened and
  * decoded tapes of at most a quarter of the pools' bytes (80 MB at most) and half
- * again on growth. This second part makes
- * level passes faster and gives way: an allocation of the context that the
- * budget would refuse takes it back first (and waits for the device), except
- * from trees whose voxelization was captured in a graph. */
+ * again on growth. This second part makes level passes faster and gives way: an
+ * allocation of the context that the budget would refuse takes it back first (and
+ * waits for the device), except from trees whose voxelization was captured in a
+ * graph. */
 frep_status frep_tree_create(frep_ctx* ctx, const frep_grid* grid, const frep_voxelize_opts* opts,
                              frep_tree** out);
 void frep_tree_destroy(frep_tree* tree);

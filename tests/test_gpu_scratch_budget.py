@@ -98,3 +98,35 @@ def test_item_room_gives_way(scene, what):
         vs.cleanup()
     assert _used(ctx) == 0
     ctx.close()
+
+
+def test_scratch_of_a_captured_voxelization_stays(scene):
+    """A graph holds the scratch's address: no other allocation takes its room."""
+    import torch
+    sc, tape, want = scene
+    big = frep.Context(0, hbm_budget_bytes=16 << 30)
+    first = []
+    pools = _grown(big, lambda: first.append(_tree(big, sc, tape, LARGE)))
+    roomy = _grown(big, lambda: frep.Voxelizer(big, first[0]).voxelize(0.0))
+    first[0].cleanup()
+    big.close()
+    ctx = frep.Context(0, hbm_budget_bytes=2 * pools + roomy - 8 * MB)
+    a = _tree(ctx, sc, tape, LARGE)
+    v = frep.Voxelizer(ctx, a)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        v.voxelize(0.0, stream=stream)
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+            v.voxelize(0.0, stream=stream)
+        before = _used(ctx)
+        with pytest.raises(frep.FrepError):
+            _tree(ctx, sc, tape, LARGE)
+        assert _used(ctx) == before
+        graph.replay()
+        stream.synchronize()
+    assert compare_trees_fast(a.export(), want) == []
+    del graph
+    a.cleanup()
+    ctx.close()
