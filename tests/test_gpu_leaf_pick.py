@@ -41,6 +41,8 @@ def _passes(call):
         for k in us:
             if e.device_type == torch.autograd.DeviceType.CUDA and k in e.name:
                 us[k] += e.time_range.end - e.time_range.start
+    if not any(us.values()):
+        pytest.skip("no kernel times: the profiler is not available")
     return us["leaf_level_kernel"], us["point_level_kernel"]
 
 
